@@ -86,80 +86,168 @@ __global__ void k_adj_deposit_grad(Parts<T> P, Mesh m, const T *__restrict__ del
     for (int k = 0; k < R; ++k) db[k][i] = (T)mass * g[k];
 }
 
-// Per-block maximum of |v| over all components.
-template <typename T>
-__global__ void k_absmax(const T *v0, const T *v1, const T *v2, size_t n, int R, double *part) {
-    __shared__ double sm[32];
-    double mx = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        mx = fmax(mx, fabs((double)v0[i]));
-        if (R > 1) mx = fmax(mx, fabs((double)v1[i]));
-        if (R > 2) mx = fmax(mx, fabs((double)v2[i]));
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, sm[w]);
-        part[blockIdx.x] = r;
-    }
+// Running maximum of |pbar|: the warps of k_adj_step reduce into ABS_SLOTS
+// slots, one 32-byte sector each (a maximum does not depend on the order), as
+// the bits of non-negative doubles, which order as integers.
+constexpr int ABS_SLOTS = 128;
+
+__device__ inline void absmax_add(unsigned long long *slots, unsigned lanes, unsigned slot, float v) {
+    const float mx = __uint_as_float(__reduce_max_sync(lanes, __float_as_uint(v)));
+    if ((threadIdx.x & 31) == 0)
+        atomicMax(slots + 4 * slot, (unsigned long long)__double_as_longlong((double)mx));
+}
+__device__ inline void absmax_add(unsigned long long *slots, unsigned lanes, unsigned slot, double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(lanes, hi);
+    const unsigned ml = __reduce_max_sync(lanes, hi == mh ? lo : 0u);
+    if ((threadIdx.x & 31) == 0) atomicMax(slots + 4 * slot, ((unsigned long long)mh << 32) | ml);
 }
 
-// Fixed-point exponent S for the vector deposit: every cell sum of
-// |v| w 2^S stays below 2^61 (gather weights with the truncating origin can
-// reach 3 per axis).
-__global__ void k_fix_exponent(const double *part, int nb, double np, int R, int *S) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double mx = 0;
-    for (int b = 0; b < nb; ++b) mx = fmax(mx, part[b]);
-    if (!(mx > 0)) {
-        *S = 0;
-        return;
+// Fixed-point exponent S for the vector deposit of values up to the slots'
+// maximum: every cell sum of |v| w 2^S stays below 2^61 (gather weights with
+// the truncating origin can reach 3 per axis). Clears the slots.
+__global__ void __launch_bounds__(ABS_SLOTS) k_fix_exponent(unsigned long long *slots, double np, int R, int *S) {
+    __shared__ unsigned long long part[ABS_SLOTS];
+    part[threadIdx.x] = slots[4 * threadIdx.x];
+    slots[4 * threadIdx.x] = 0ull;
+    for (int h = ABS_SLOTS / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if ((int)threadIdx.x < h) part[threadIdx.x] = max(part[threadIdx.x], part[threadIdx.x + h]);
     }
-    double lg = log2(mx) + log2(np) + 2.0 * R;
-    int s = (int)floor(61.0 - lg);
-    *S = max(-1000, min(1000, s));
+    if (threadIdx.x != 0) return;
+    const double mx = __longlong_as_double((long long)part[0]);
+    int s = 0;
+    if (mx > 0) {
+        const double lg = log2(mx) + log2(np) + 2.0 * R;
+        s = max(-1000, min(1000, (int)floor(61.0 - lg)));
+    }
+    *S = s;
 }
 
 // U_k(c) += v_k W^g_b for every particle and gather corner, in 64-bit
 // fixed point (integer atomics: the sums are exact and order-independent).
-template <typename T, int R>
-__global__ void k_adj_vec_deposit(Parts<T> P, Mesh m, const T *v0, const T *v1, const T *v2, int periodic,
-                                  const int *__restrict__ S, unsigned long long *U0, unsigned long long *U1,
-                                  unsigned long long *U2) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.np) return;
+// Bound by the load/store units' and L2's 64-bit reductions (2^R R adds of 8
+// bytes per particle). MERGE: fewer of them reach the L2. One thread takes
+// two particles that follow each other along the slowest axis; where the
+// second sits one cell further along that axis, the first's upper corners are
+// the second's lower ones and their integers are added in registers. Likewise
+// along x: a lane whose origin is one cell beyond the lane before it adds that
+// lane's upper-x values (shuffles) to its own lower-x ones. Integer sums, so
+// the same bits. 256^3 particles, a = 0.3: 795 -> 600 us; without the x
+// merge 690, with four or eight particles per thread 650, one 640.
+template <typename T, int R, bool MERGE>
+__global__ void __launch_bounds__(256)
+    k_adj_vec_deposit(Parts<T> P, Mesh m, const T *__restrict__ v0, const T *__restrict__ v1, const T *__restrict__ v2,
+                      int periodic, const int *__restrict__ S, unsigned long long *U0, unsigned long long *U1,
+                      unsigned long long *U2) {
+    constexpr int NZ = MERGE ? 2 : 1;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= P.np / NZ) return;
+    const int ls = (R - 1) * P.mshift;  // log2 of the particles per layer of the slowest axis
+    const size_t i0 = (t & (((size_t)1 << ls) - 1)) | ((t >> ls) * NZ << ls);
     const T *vv[3] = {v0, v1, v2};
-    unsigned long long *U[3] = {U0, U1, U2};
-    int q[3], o[3];
-    T a0[3], a1[3], v[3];
-    lattice<T, R>(P, i, q);
+    const size_t cb = cell_base(P, m, i0);  // the NZ particles belong to one member
+    unsigned long long *U[3] = {U0 + cb, U1 + cb, U2 + cb};
+    const double sc = ldexp(1.0, *S);  // a power of two: v z sc is exact in double for FP32
+    // rn(x sc): for 2^18 particles and more the fixed-point exponent keeps
+    // |x sc| below 2^43, so one fused multiply-add onto 1.5 2^52 leaves the
+    // rounded integer in the mantissa (the conversion instruction runs at a
+    // quarter of that rate)
+    auto fix = [&](double x) -> long long {
+        if constexpr (MERGE)
+            return __double_as_longlong(__fma_rn(x, sc, 6755399441055744.0)) - 0x4338000000000000LL;
+        else
+            return __double2ll_rn(x * sc);
+    };
+    constexpr int HALF = 1 << (R - 1);
+    auto emit = [&](const int *o, int b, const long long *q) {
+        const uint32_t ci = corner_index<R>(o, b, m);
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-        gather_axis<T>(P.d[k][i], q[k], periodic != 0, &o[k], &a1[k]);
-        a0[k] = T(1) - a1[k];
-        v[k] = vv[k][i];
-    }
-    const int s = *S;
+        for (int k = 0; k < R; ++k)
+            if (q[k]) atomicAdd(U[k] + ci, (unsigned long long)q[k]);
+    };
+    int po[3] = {0, 0, 0};
+    long long pend[HALF][R];
 #pragma unroll
-    for (int b = 0; b < (1 << R); ++b) {
-        T z = 1;
-#pragma unroll
-        for (int k = 0; k < R; ++k) z *= ((b >> k) & 1) ? a1[k] : a0[k];
-        size_t ci = cell_base(P, m, i) + corner_index<R>(o, b, m);
+    for (int j = 0; j < NZ; ++j) {
+        const size_t i = i0 + ((size_t)j << ls);
+        int q[3], o[3] = {0, 0, 0};
+        T a0[3], a1[3], v[3];
+        lattice<T, R>(P, i, q);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
-            long long qv = __double2ll_rn(ldexp((double)v[k] * (double)z, s));
-            if (qv) atomicAdd(U[k] + ci, (unsigned long long)qv);
+            gather_axis<T>(P.d[k][i], q[k], periodic != 0, &o[k], &a1[k]);
+            a0[k] = T(1) - a1[k];
+            v[k] = vv[k][i];
         }
+        bool meet = j > 0 && o[R - 1] == po[R - 1] + 1;
+#pragma unroll
+        for (int k = 0; k < R - 1; ++k) meet = meet && o[k] == po[k];
+        // the lane before this one sits one cell back along x: its
+        // upper-x corners are this lane's lower-x corners
+        bool take = false, give = false;
+        if constexpr (MERGE) {
+            take = (threadIdx.x & 31) != 0;
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int ok = __shfl_up_sync(FULL, o[k], 1);
+                take = take && ok + (k == 0 ? 1 : 0) == o[k];
+            }
+            give = __shfl_down_sync(FULL, (int)take, 1) != 0 && (threadIdx.x & 31) != 31;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // the lower, then the upper layer
+            long long w[HALF][R];
+#pragma unroll
+            for (int b = 0; b < HALF; ++b) {
+                const int c = h * HALF + b;
+                T z = 1;
+#pragma unroll
+                for (int k = 0; k < R; ++k) z *= ((c >> k) & 1) ? a1[k] : a0[k];
+#pragma unroll
+                for (int k = 0; k < R; ++k) w[b][k] = fix((double)v[k] * (double)z);
+            }
+            if (h == 0 && j > 0) {
+                if (meet) {
+#pragma unroll
+                    for (int b = 0; b < HALF; ++b)
+#pragma unroll
+                        for (int k = 0; k < R; ++k) w[b][k] += pend[b][k];
+                } else {
+#pragma unroll
+                    for (int b = 0; b < HALF; ++b) emit(po, HALF + b, pend[b]);
+                }
+            }
+            if (h == 0 || j + 1 == NZ) {
+                if constexpr (MERGE) {
+#pragma unroll
+                    for (int b = 0; b < HALF; b += 2)
+#pragma unroll
+                        for (int k = 0; k < R; ++k) {
+                            const long long u = __shfl_up_sync(FULL, w[b + 1][k], 1);
+                            if (take) w[b][k] += u;
+                        }
+                }
+#pragma unroll
+                for (int b = 0; b < HALF; ++b)
+                    if (!MERGE || !(b & 1) || !give) emit(o, h * HALF + b, w[b]);
+            } else {
+#pragma unroll
+                for (int b = 0; b < HALF; ++b)
+#pragma unroll
+                    for (int k = 0; k < R; ++k) pend[b][k] = w[b][k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k) po[k] = o[k];
     }
 }
 
 // out(c) = -sum_k FD4_k(U_k)(c): the adjoint of the FD4 gradient, from the
 // fixed-point meshes (scale 2^-S) or from real meshes (S == nullptr).
 template <typename T, int R, typename UT>
-__global__ void k_neg_div(const UT *U0, const UT *U1, const UT *U2, const int *S, T *out, Mesh m) {
+__global__ void k_neg_div(const UT *__restrict__ U0, const UT *__restrict__ U1, const UT *__restrict__ U2,
+                          const int *__restrict__ S, T *__restrict__ out, Mesh m) {
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.cells) return;
     const UT *U[3] = {U0, U1, U2};
@@ -182,14 +270,85 @@ __global__ void k_neg_div(const UT *U0, const UT *U1, const UT *U2, const int *S
     out[c] = (T)(-acc * sc);
 }
 
+// 12 FD4 of the values at -2, -1, 1, 2 of a line. Fixed-point values are
+// combined as integers: the exponent keeps a component's sum over all cells
+// below 2^60, so |u(-2) - u(2) + 8 (u(1) - u(-1))| < 2^63 for four distinct
+// cells: exact, and one conversion instead of four.
+__device__ inline double fd4_x12(unsigned long long m2, unsigned long long m1, unsigned long long p1,
+                                 unsigned long long p2) {
+    return (double)(long long)((m2 - p2) + ((p1 - m1) << 3));
+}
+template <typename T> __device__ inline double fd4_x12(T m2, T m1, T p1, T p2) {
+    return ((double)m2 - (double)p2) + 8.0 * ((double)p1 - (double)m1);
+}
+
+// The same for 3D meshes of 32 cells per side and more: a block of 32 x 8
+// threads marches NDZ planes along z, so that each thread keeps its column's
+// five U2 values in registers and the rows it reads for y stay in L1. Bound
+// by the L2 reads of the thread-per-cell form (nine mesh values per cell
+// instead of three); fixed-point meshes, 128^3 21 -> 14 us, 256^3 161 -> 114
+// (with 16 planes 24 and 125, with 4 14 and 110 but 126 instead of 82 us for
+// real meshes).
+constexpr int NDZ = 8;
+template <typename T, typename UT>
+__global__ void __launch_bounds__(256)
+    k_neg_div_z(const UT *__restrict__ U0, const UT *__restrict__ U1, const UT *__restrict__ U2,
+                const int *__restrict__ S, T *__restrict__ out, Mesh m) {
+    const uint32_t mask = (uint32_t)m.n - 1;
+    const int s = m.shift;
+    unsigned b = blockIdx.x;
+    const uint32_t x = (b & ((1u << (s - 5)) - 1)) * 32 + (threadIdx.x & 31);
+    b >>= s - 5;
+    const uint32_t y = (b & ((1u << (s - 3)) - 1)) * 8 + (threadIdx.x >> 5);
+    b >>= s - 3;
+    const uint32_t nz = (unsigned)m.n / NDZ;
+    const uint32_t z0 = (b & (nz - 1)) * NDZ;
+    const size_t mb = (size_t)(b / nz) << m.cshift;
+    U0 += mb;
+    U1 += mb;
+    U2 += mb;
+    out += mb;
+    const uint32_t col = (y << s) | x;
+    uint32_t rx[5], ry[5];  // offsets of the x and y neighbours in a plane
+#pragma unroll
+    for (int o = 0; o < 5; ++o) {
+        rx[o] = (y << s) | ((x + o - 2) & mask);
+        ry[o] = (((y + o - 2) & mask) << s) | x;
+    }
+    auto plane = [&](uint32_t z) { return (z & mask) << (2 * s); };
+    UT q[5];  // this column at z - 2 .. z + 2
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = __ldg(U2 + (plane(z0 + j - 2) | col));
+    const double sc = (S ? ldexp(1.0, -*S) : 1.0) * (-1.0 / 12.0);
+#pragma unroll 4
+    for (int zi = 0; zi < NDZ; ++zi) {
+        const uint32_t z = z0 + zi, pz = plane(z);
+        q[4] = __ldg(U2 + (plane(z + 2) | col));
+        const UT *__restrict__ a = U0 + pz, *__restrict__ c = U1 + pz;
+        double acc = fd4_x12(__ldg(a + rx[0]), __ldg(a + rx[1]), __ldg(a + rx[3]), __ldg(a + rx[4]));
+        acc += fd4_x12(__ldg(c + ry[0]), __ldg(c + ry[1]), __ldg(c + ry[3]), __ldg(c + ry[4]));
+        acc += fd4_x12(q[0], q[1], q[3], q[4]);
+        out[pz | col] = (T)(acc * sc);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[j] = q[j + 1];
+    }
+}
+
 // One adjoint step (see the file comment): updates dbar, pbar and runs the
 // state back from s_{i+1} to s_i, using G = FD4 gradient at d_{i+1} and
-// rhobar = Green * div.
+// rhobar = Green * div (null: zero); the maximum of the new |pbar| goes into
+// absmax (a pass of its own over pbar before: 160 us per step at 256^3).
+// Bound by the chain of its twelve streams and 16 corner loads: the register
+// budget of four blocks per SM takes 450 us at 256^3, three 547, five 524;
+// walking the lattice in 16 x 4 x 4 tiles 578 (half-used sectors of the
+// streams cost more than the corner reads' locality gains), streaming loads
+// and stores 457.
 template <typename T, int R>
-__global__ void k_adj_step(Parts<T> P, Mesh m, const G4<T> *__restrict__ G, const T *__restrict__ rhobar,
-                           T *pb0, T *pb1, T *pb2, T *db0, T *db1, T *db2, double ck, double cd, double mass,
-                           int periodic) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256, 4)
+    k_adj_step(Parts<T> P, Mesh m, const G4<T> *__restrict__ G, const T *__restrict__ rhobar, T *pb0, T *pb1, T *pb2,
+               T *db0, T *db1, T *db2, double ck, double cd, double mass, int periodic, unsigned long long *absmax) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lanes = __ballot_sync(FULL, i < P.np);
     if (i >= P.np) return;
     T *pbv[3] = {pb0, pb1, pb2}, *dbv[3] = {db0, db1, db2};
     T d[3], p[3], v[3], dbar[3];
@@ -211,7 +370,6 @@ __global__ void k_adj_step(Parts<T> P, Mesh m, const G4<T> *__restrict__ G, cons
     T F[3] = {T(0), T(0), T(0)}, t1[3] = {T(0), T(0), T(0)}, t2[3] = {T(0), T(0), T(0)};
     const size_t cb = cell_base(P, m, i);
     G += cb;
-    rhobar += cb;
 #pragma unroll
     for (int b = 0; b < (1 << R); ++b) {
         G4<T> g = load_g4(G + corner_index<R>(o, b, m));
@@ -228,23 +386,30 @@ __global__ void k_adj_step(Parts<T> P, Mesh m, const G4<T> *__restrict__ G, cons
             t1[k] += dweight<T, R>(a0, a1, b, k) * vg;
         }
     }
-    deposit_corner_frame<T, R>(P, m, i, d, cell, b0, b1);
+    if (rhobar) {
+        rhobar += cb;
+        deposit_corner_frame<T, R>(P, m, i, d, cell, b0, b1);
 #pragma unroll
-    for (int b = 0; b < (1 << R); ++b) {
-        T r = __ldg(rhobar + corner_index<R>(cell, b, m));
+        for (int b = 0; b < (1 << R); ++b) {
+            T r = __ldg(rhobar + corner_index<R>(cell, b, m));
 #pragma unroll
-        for (int k = 0; k < R; ++k) t2[k] += dweight<T, R>(b0, b1, b, k) * r;
+            for (int k = 0; k < R; ++k) t2[k] += dweight<T, R>(b0, b1, b, k) * r;
+        }
     }
+    T mx = T(0);
     const T tck = (T)ck, tcd = (T)cd, tm = (T)mass;
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         T dbn = dbar[k] - tck * (t1[k] + tm * t2[k]);
+        T pbn = v[k] + tcd * dbn;
         dbv[k][i] = dbn;
-        pbv[k][i] = v[k] + tcd * dbn;
+        pbv[k][i] = pbn;
+        mx = fmax(mx, fabs(pbn));
         T pold = p[k] + tck * F[k];
         P.p[k][i] = pold;
         P.d[k][i] = d[k] - tcd * pold;
     }
+    absmax_add(absmax, lanes, (blockIdx.x * 8 + (threadIdx.x >> 5)) % ABS_SLOTS, mx);
 }
 
 // ubar_k = cdz dbar_k + cpz pbar_k in place in dbar (particle i = mass cell i).
@@ -277,7 +442,8 @@ template <typename T, int R> struct Diff : DiffBase {
     T *db[3] = {nullptr, nullptr, nullptr}, *pb[3] = {nullptr, nullptr, nullptr};
     unsigned long long *U[3] = {nullptr, nullptr, nullptr};
     T *rhobar = nullptr;
-    int *S = nullptr;
+    int *S = nullptr;           // fixed-point exponent of the vector deposit
+    unsigned long long *absmax = nullptr;  // slots of the running |pbar| maximum
     std::vector<T *> ckpt;  // per checkpoint: d[0..R), p[0..R)
     std::vector<double> a_start;
     cudaEvent_t ev = nullptr;
@@ -315,6 +481,7 @@ template <typename T, int R> struct Diff : DiffBase {
         }
         CONAN_TRY(pm.alloc(&rhobar, pm.mf.cells));
         CONAN_TRY(pm.alloc(&S, 1));
+        CONAN_TRY(pm.alloc(&absmax, 4 * ABS_SLOTS));
         unsigned k = p.checkpoint_every ? p.checkpoint_every : 1;
         for (unsigned i = 0; i <= p.n; i += k)
             for (int c = 0; c < 2 * R; ++c) {
@@ -409,18 +576,53 @@ template <typename T, int R> struct Diff : DiffBase {
         return leave(stream);
     }
 
+    template <typename UT> int neg_div(UT *const *u, const int *exps, T *out, const Mesh &m) {
+        if constexpr (R == 3) {
+            if (m.n >= 32) {
+                const unsigned blocks = (unsigned)((size_t)(m.n / 32) * (m.n / 8) * (m.n / NDZ) * m.batch);
+                k_neg_div_z<T, UT><<<blocks, 256, 0, pm.st>>>(u[0], u[1], u[2], exps, out, m);
+                CONAN_LAUNCHED();
+                return CONAN_OK;
+            }
+        }
+        k_neg_div<T, R, UT><<<(unsigned)((m.cells + 255) / 256), 256, 0, pm.st>>>(u[0], u[1], u[2], exps, out, m);
+        CONAN_LAUNCHED();
+        return CONAN_OK;
+    }
+
     // rhobar = Green(a) * (-sum_k FD4_k(U_k)) without touching the gradient mesh
     int adjoint_poisson(double am) {
-        cudaStream_t st = pm.st;
-        const Mesh &mf = pm.mf;
-        unsigned gc = (unsigned)((mf.cells + 255) / 256);
-        k_neg_div<T, R, unsigned long long><<<gc, 256, 0, st>>>(U[0], U[1], U[2], S, rhobar, mf);
-        CONAN_LAUNCHED();
-        // per-member normalisation: 1 / (cells of one box)
-        double gsc = -pm.G / (am * (double)((size_t)1 << mf.cshift)) * std::pow(prm.pm.size / (2 * M_PI), 2);
+        CONAN_TRY(neg_div(U, S, rhobar, pm.mf));
+        const double gsc = pm.poisson_scale(am);
+        if constexpr (sizeof(T) == 4) {
+            if (pm.zpass) {  // the forward solve's plane transforms and z pass
+                CONAN_TRY(pm.fft2.forward(rhobar, pm.spec));
+                CONAN_TRY(pm.green_z(gsc));
+                CONAN_TRY(pm.fft2.inverse(pm.spec, rhobar));
+                return CONAN_OK;
+            }
+        }
         CONAN_TRY(pm.fft.forward(rhobar, pm.spec));
         CONAN_TRY(pm.green(pm.spec, gsc));
         CONAN_TRY(pm.fft.inverse(pm.spec, rhobar));
+        return CONAN_OK;
+    }
+
+    // U = gather-transpose deposit of pb. The merging kernel needs whole warps
+    // within one member (8 particles per side) and, for its one-instruction rounding, a fixed-point
+    // exponent that leaves particles below 2^51 units: 2^18 particles are
+    // enough for both (and smaller lattices are launch-bound either way).
+    int vec_deposit() {
+        cudaStream_t st = pm.st;
+        if (R > 1 && mm.n >= 8 && pm.np >= ((size_t)1 << 18)) {
+            const size_t nt = pm.np / 2;
+            k_adj_vec_deposit<T, R, (R > 1)><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(
+                pm.P, pm.mf, pb[0], pb[1], pb[2], prm.pm.periodic_gather, S, U[0], U[1], U[2]);
+        } else {
+            k_adj_vec_deposit<T, R, false><<<gp(), 256, 0, st>>>(pm.P, pm.mf, pb[0], pb[1], pb[2],
+                                                                 prm.pm.periodic_gather, S, U[0], U[1], U[2]);
+        }
+        CONAN_LAUNCHED();
         return CONAN_OK;
     }
 
@@ -435,25 +637,27 @@ template <typename T, int R> struct Diff : DiffBase {
         k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, rhobar, pm.mass, db[0], db[1], db[2]);
         CONAN_LAUNCHED();
         for (int k = 0; k < R; ++k) CONAN_CUDA(cudaMemsetAsync(pb[k], 0, pm.np * sizeof(T), st));
+        // the previous backward's first step left its maximum behind
+        CONAN_CUDA(cudaMemsetAsync(absmax, 0, 4 * ABS_SLOTS * sizeof(unsigned long long), st));
         for (int i = (int)prm.n - 1; i >= 0; --i) {
             double a = a_start[i], am = a + prm.da / 2;
             double ck = pm.coef_kick(am, prm.da), cd = pm.coef_drift(a, prm.da);
             // forward force at d_{i+1}: deposit, potential, gradient mesh
             CONAN_TRY(pm.deposit_poisson(am));
-            // U = gather-transpose deposit of v = pbar
-            const int nb = 296;
-            k_absmax<T><<<nb, 256, 0, st>>>(pb[0], pb[1], pb[2], pm.np, R, part);
-            CONAN_LAUNCHED();
-            k_fix_exponent<<<1, 32, 0, st>>>(part, nb, (double)pm.np, R, S);
-            CONAN_LAUNCHED();
-            for (int k = 0; k < R; ++k)
-                CONAN_CUDA(cudaMemsetAsync(U[k], 0, mf.cells * sizeof(unsigned long long), st));
-            k_adj_vec_deposit<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, pb[0], pb[1], pb[2], prm.pm.periodic_gather, S,
-                                                          U[0], U[1], U[2]);
-            CONAN_LAUNCHED();
-            CONAN_TRY(adjoint_poisson(am));
-            k_adj_step<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, pm.grad, rhobar, pb[0], pb[1], pb[2], db[0], db[1],
-                                                   db[2], ck, cd, pm.mass, prm.pm.periodic_gather);
+            // U = gather-transpose deposit of v = pbar and the density's
+            // adjoint rhobar; pbar is zero in the last step (the loss sees
+            // positions only), and so is rhobar
+            const bool vz = i == (int)prm.n - 1;
+            if (!vz) {
+                k_fix_exponent<<<1, ABS_SLOTS, 0, st>>>(absmax, (double)pm.np, R, S);
+                CONAN_LAUNCHED();
+                for (int k = 0; k < R; ++k)
+                    CONAN_CUDA(cudaMemsetAsync(U[k], 0, mf.cells * sizeof(unsigned long long), st));
+                CONAN_TRY(vec_deposit());
+                CONAN_TRY(adjoint_poisson(am));
+            }
+            k_adj_step<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, pm.grad, vz ? nullptr : rhobar, pb[0], pb[1], pb[2],
+                                                   db[0], db[1], db[2], ck, cd, pm.mass, prm.pm.periodic_gather, absmax);
             CONAN_LAUNCHED();
             if ((unsigned)i % kev() == 0) CONAN_TRY(load_ckpt((unsigned)i / kev()));
         }
@@ -463,8 +667,7 @@ template <typename T, int R> struct Diff : DiffBase {
             k_za_adjoint<T><<<gm, 256, 0, st>>>(db[k], pb[k], mm.cells, cdz(), cpz());
             CONAN_LAUNCHED();
         }
-        k_neg_div<T, R, T><<<gm, 256, 0, st>>>(db[0], db[1], db[2], nullptr, ict, mm);
-        CONAN_LAUNCHED();
+        CONAN_TRY(neg_div(db, nullptr, ict, mm));
         for (int b = 0; b < mm.batch; ++b) {
             const size_t o = member_cells(mm, b);
             CONAN_TRY(potential_device<T>(mm1, ic[b].size, ict + o, ics, icfft, st));
