@@ -448,6 +448,9 @@ template <typename T, int R> struct Diff : DiffBase {
     std::vector<double> a_start;
     cudaEvent_t ev = nullptr;
     bool have_forward = false;
+    // the gradient mesh is that of the final positions (forward's last step), as
+    // backward's first step needs it
+    bool grad_final = false;
 
     ~Diff() override {
         if (pm.st) cudaStreamSynchronize(pm.st);
@@ -518,13 +521,11 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_CUDA(cudaStreamSynchronize(pm.st));
         return pm.check_err();
     }
-    int save_ckpt(unsigned slot) {
-        for (int k = 0; k < R; ++k) {
-            CONAN_CUDA(cudaMemcpyAsync(ckpt[slot * 2 * R + k], pm.P.d[k], pm.np * sizeof(T), cudaMemcpyDeviceToDevice,
-                                       pm.st));
-            CONAN_CUDA(cudaMemcpyAsync(ckpt[slot * 2 * R + R + k], pm.P.p[k], pm.np * sizeof(T),
-                                       cudaMemcpyDeviceToDevice, pm.st));
-        }
+    // Positions (mom = false) or momenta of the current state into a slot.
+    int save_ckpt(unsigned slot, bool mom) {
+        for (int k = 0; k < R; ++k)
+            CONAN_CUDA(cudaMemcpyAsync(ckpt[slot * 2 * R + (mom ? R : 0) + k], mom ? pm.P.p[k] : pm.P.d[k],
+                                       pm.np * sizeof(T), cudaMemcpyDeviceToDevice, pm.st));
         return CONAN_OK;
     }
     int load_ckpt(unsigned slot) {
@@ -544,11 +545,11 @@ template <typename T, int R> struct Diff : DiffBase {
     // the Zel'dovich start of the particle state at (a0, a0 + da/2).
     int initial_state(const void *noise) {
         cudaStream_t st = pm.st;
+        grad_final = false;
         CONAN_CUDA(cudaMemcpyAsync(w, noise, mm.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        CONAN_CUDA(cudaMemcpyAsync(ict, w, mm.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
         for (int b = 0; b < mm.batch; ++b) {  // initial conditions, member by member
             T *x = ict + member_cells(mm, b);
-            CONAN_TRY(grf_device<T>(ic[b], mm1, x, ics, icfft, part, st));
+            CONAN_TRY(grf_device<T>(ic[b], mm1, w + member_cells(mm, b), x, ics, icfft, part, st));
             CONAN_TRY(potential_device<T>(mm1, ic[b].size, x, ics, icfft, st));
         }
         k_zeldovich<T, R><<<gp(), 256, 0, st>>>(pm.P, ict, mm, cdz(), cpz());
@@ -561,17 +562,26 @@ template <typename T, int R> struct Diff : DiffBase {
 
     int forward(const void *noise, void *density, void *stream) override {
         CONAN_TRY(enter(stream));
-        cudaStream_t st = pm.st;
         CONAN_TRY(initial_state(noise));
+        // The kick of a step and the drift (with its deposit) of the next are
+        // one launch, as in a run; a checkpoint between them takes the
+        // positions before it (a kick moves none) and the momenta after it
+        // (a drift changes none).
+        CONAN_TRY(save_ckpt(0, false));
+        CONAN_TRY(save_ckpt(0, true));
+        CONAN_TRY(pm.gkd(false, 0, true, pm.coef_drift(a_start[0], prm.da), true));
         for (unsigned i = 0; i < prm.n; ++i) {
-            if (i % kev() == 0) CONAN_TRY(save_ckpt(i / kev()));
-            double a = a_start[i], am = a + prm.da / 2;
-            CONAN_TRY(pm.gkd(false, 0, true, pm.coef_drift(a, prm.da), true));
-            CONAN_TRY(pm.deposit_poisson(am));
-            CONAN_TRY(pm.gkd(true, pm.coef_kick(am, prm.da), false, 0, false));
+            const double am = a_start[i] + prm.da / 2;
+            const bool last = i + 1 == prm.n, save = !last && (i + 1) % kev() == 0;
+            // the positions of the last deposit are the final ones: its
+            // density is the output
+            CONAN_TRY(pm.deposit_poisson(am, last ? (T *)density : nullptr));
+            if (save) CONAN_TRY(save_ckpt((i + 1) / kev(), false));
+            CONAN_TRY(pm.gkd(true, pm.coef_kick(am, prm.da), !last, last ? 0 : pm.coef_drift(a_start[i + 1], prm.da),
+                             !last));
+            if (save) CONAN_TRY(save_ckpt((i + 1) / kev(), true));
         }
-        CONAN_TRY(pm.deposit());  // final density
-        CONAN_CUDA(cudaMemcpyAsync(density, pm.mesh, pm.mf.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
+        grad_final = true;
         have_forward = true;
         return leave(stream);
     }
@@ -633,8 +643,7 @@ template <typename T, int R> struct Diff : DiffBase {
         const Mesh &mf = pm.mf;
         const unsigned gc = (unsigned)((mf.cells + 255) / 256);
         // the density adjoint through the final deposit
-        CONAN_CUDA(cudaMemcpyAsync(rhobar, gdens, mf.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, rhobar, pm.mass, db[0], db[1], db[2]);
+        k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, (const T *)gdens, pm.mass, db[0], db[1], db[2]);
         CONAN_LAUNCHED();
         for (int k = 0; k < R; ++k) CONAN_CUDA(cudaMemsetAsync(pb[k], 0, pm.np * sizeof(T), st));
         // the previous backward's first step left its maximum behind
@@ -643,7 +652,9 @@ template <typename T, int R> struct Diff : DiffBase {
             double a = a_start[i], am = a + prm.da / 2;
             double ck = pm.coef_kick(am, prm.da), cd = pm.coef_drift(a, prm.da);
             // forward force at d_{i+1}: deposit, potential, gradient mesh
-            CONAN_TRY(pm.deposit_poisson(am));
+            // (the forward pass leaves the last step's)
+            if (!grad_final) CONAN_TRY(pm.deposit_poisson(am));
+            grad_final = false;
             // U = gather-transpose deposit of v = pbar and the density's
             // adjoint rhobar; pbar is zero in the last step (the loss sees
             // positions only), and so is rhobar

@@ -191,12 +191,13 @@ template <typename T> struct ICWork {
     }
 };
 
-// Device pipeline of _generate_random_field<R>, src/ic/ic.cc:37-98, on an
-// already filled real mesh `mesh` (the noise); leaves the density in it.
+// Device pipeline of _generate_random_field<R>, src/ic/ic.cc:37-98, from the
+// real mesh `noise` (an out-of-place R2C leaves its input alone) to the
+// density in `mesh`.
 template <typename T>
-int grf_device(const conan_ic_params &p, const Mesh &m, T *mesh, typename Cplx<T>::type *spec, FFTPair &fft,
-               double *part, cudaStream_t st) {
-    CONAN_TRY(fft.forward(mesh, spec));
+int grf_device(const conan_ic_params &p, const Mesh &m, T *noise, T *mesh, typename Cplx<T>::type *spec,
+               FFTPair &fft, double *part, cudaStream_t st) {
+    CONAN_TRY(fft.forward(noise, spec));
     ICFilter F{};
     F.ns = p.ns;
     F.L = p.size;
@@ -228,9 +229,9 @@ int grf_device(const conan_ic_params &p, const Mesh &m, T *mesh, typename Cplx<T
     CONAN_TRY(fft.inverse(spec, mesh));
     return CONAN_OK;
 }
-template int grf_device<float>(const conan_ic_params &, const Mesh &, float *, cufftComplex *, FFTPair &,
+template int grf_device<float>(const conan_ic_params &, const Mesh &, float *, float *, cufftComplex *, FFTPair &,
                                double *, cudaStream_t);
-template int grf_device<double>(const conan_ic_params &, const Mesh &, double *, cufftDoubleComplex *,
+template int grf_device<double>(const conan_ic_params &, const Mesh &, double *, double *, cufftDoubleComplex *,
                                 FFTPair &, double *, cudaStream_t);
 
 // _compute_potential<R>, src/ic/ic.cc:100-117, in place on a device mesh.
@@ -377,7 +378,7 @@ template <typename T> int ic_generate(const conan_ic_params &p, const double *no
         CONAN_TRY(w.upload(noise));
     else
         CONAN_TRY(noise_device<T>(w.m, p.seed, w.mesh, w.st));
-    CONAN_TRY(grf_device<T>(p, w.m, w.mesh, w.spec, w.fft, w.part, w.st));
+    CONAN_TRY(grf_device<T>(p, w.m, w.mesh, w.mesh, w.spec, w.fft, w.part, w.st));
     return w.download(out);
 }
 

@@ -22,9 +22,9 @@ int check_ic_params(const conan_ic_params *p);
 
 // Philox white noise into a device mesh.
 template <typename T> int noise_device(const Mesh &m, unsigned long long seed, T *mesh, cudaStream_t st);
-// Noise mesh -> density mesh, in place (uses spec as scratch).
+// Noise mesh (kept) -> density mesh (may be the same; uses spec as scratch).
 template <typename T>
-int grf_device(const conan_ic_params &p, const Mesh &m, T *mesh, typename Cplx<T>::type *spec, FFTPair &fft,
+int grf_device(const conan_ic_params &p, const Mesh &m, T *noise, T *mesh, typename Cplx<T>::type *spec, FFTPair &fft,
                double *part, cudaStream_t st);
 // Adjoint of grf_device: dL/dw from dL/d(density) (dbar is overwritten).
 template <typename T>

@@ -478,11 +478,17 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
-    int deposit_lag() {
-        CONAN_TRY(lag_accumulate());
+    // The accumulator's density contrast into out.
+    int acc_mesh(T *out) {
         size_t nt = (mf.cells + 3) / 4;  // four cells per thread
         CONAN_TIMED(prof, "deposit_mesh", st,
-                    (k_acc_mesh<T><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(lacc, mesh, mf.cells, mass)));
+                    (k_acc_mesh<T><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(lacc, out, mf.cells, mass)));
+        return CONAN_OK;
+    }
+
+    int deposit_lag() {
+        CONAN_TRY(lag_accumulate());
+        CONAN_TRY(acc_mesh(mesh));
         CONAN_TIMED(prof, "deposit_clear", st,
                     CONAN_CUDA(cudaMemsetAsync(lacc, 0, mf.cells * sizeof(unsigned long long), st)));
         mesh_holds = 1;
@@ -772,9 +778,11 @@ template <typename T, int R> struct PM : PMBase {
     // The deposit of the current positions and the Poisson solve of the
     // kick that follows it: through the cluster plane pass when it is on,
     // else deposit() (density mesh) and poisson().
-    int deposit_poisson(double a) {
+    // delta_out (device, may be null) receives the density contrast.
+    int deposit_poisson(double a, T *delta_out = nullptr) {
         if (plane_on()) {
             CONAN_TRY(lag_accumulate());
+            if (delta_out) CONAN_TRY(acc_mesh(delta_out));
             const double gs = poisson_scale(a);
             if (mf.n == 512) CONAN_TRY((plane_kc == 16 ? plane_run<512, 16>(gs) : plane_run<512, 32>(gs)));
             else CONAN_TRY((plane_kc == 16 ? plane_run<256, 16>(gs) : plane_run<256, 32>(gs)));
@@ -783,6 +791,8 @@ template <typename T, int R> struct PM : PMBase {
             return CONAN_OK;
         }
         CONAN_TRY(deposit());
+        if (delta_out)
+            CONAN_CUDA(cudaMemcpyAsync(delta_out, mesh, mf.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
         return poisson(a);
     }
 
