@@ -473,7 +473,7 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_TRY(pm.alloc(&ict2, mm.cells));
         CONAN_TRY(pm.alloc(&ics, mm.spec));
         CONAN_TRY(pm.alloc(&ics2, mm.spec));
-        CONAN_TRY(pm.alloc(&part, 1024));
+        CONAN_TRY(pm.alloc(&part, ic_scratch(mm1)));
         CONAN_TRY(icfft.create(mm1, sizeof(T) == 8, 1));
         CONAN_TRY(pm.alloc((char **)&icwork, icfft.work_bytes ? icfft.work_bytes : 16));
         CONAN_TRY(icfft.bind(icwork, pm.st));

@@ -18,6 +18,22 @@ struct ICFilter {
     double h;       // H0 / 100 (CDM branch)
 };
 
+// FP64 scratch of the field functions below (`part`): the partial sums of
+// IC_BLOCKS blocks, a few scalars behind them, and from IC_PART on the filter
+// tables of the meshes that use them: 3D, IC_TABLE_N cells per side and more
+// (an eighth of the modes' values; below that a launch costs more than the
+// values, and in 2D a quarter of few modes).
+constexpr int IC_BLOCKS = 512, IC_PART = 1024, IC_TABLE_N = 32;
+enum { IC_VAR = 0, IC_AMP, IC_SCALE, IC_DOT };  // scalars at part + IC_BLOCKS
+inline size_t ic_table_values(const Mesh &m) {
+    const size_t h = m.n / 2 + 1;
+    return m.R == 3 && m.n >= IC_TABLE_N ? h * h * h : 0;
+}
+inline size_t ic_scratch(const Mesh &m) {
+    const size_t np = ic_table_values(m);
+    return IC_PART + (np ? np + m.n / 2 + 1 : 0);
+}
+
 int check_ic_params(const conan_ic_params *p);
 
 // Philox white noise into a device mesh.
