@@ -591,12 +591,7 @@ struct FofEngine {
         return CONAN_OK;
     }
 
-    void scan(uint32_t *cnt, size_t m, uint32_t *out, cudaStream_t s) {
-        const size_t nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
-        k_scan_partial<<<(unsigned)nb, SCAN_T, 0, s>>>(cnt, m, bsum);
-        k_scan_blocks<<<1, 1024, 0, s>>>(bsum, (int)nb);
-        k_scan_final<<<(unsigned)nb, SCAN_T, 0, s>>>(cnt, m, bsum, out);
-    }
+    void scan(uint32_t *cnt, size_t m, uint32_t *out, cudaStream_t s) { scan_exclusive(cnt, m, bsum, out, s); }
 
     // Groups of the positions in Xd (device, n x R doubles); tags into tg
     // (device, n values). Enqueued on `s`; the group count is read back.

@@ -186,6 +186,7 @@ template <typename T, int R> struct PM : PMBase {
         CONAN_TRY(alloc(&err, 1));
         CONAN_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
         CONAN_CUDA(cudaMemsetAsync(count, 0, mf.cells * sizeof(uint32_t), st));
+        dep_variant = dep_default();
         bool lag = sizeof(T) == 4 && (lag_try<0>() || lag_try<1>() || lag_try<2>());
         // On fine meshes (f >= 2) a window that fits shared memory only fits
         // a small tile and holds many cells per particle, each of which gets
@@ -499,7 +500,7 @@ template <typename T, int R> struct PM : PMBase {
     int set_deposit(int mode) override {
         CONAN_TRY(drop_lag_deposit());  // a pending fused deposit belongs to the old mode
         if (mode == CONAN_DEPOSIT_SORTED) {
-            dep_variant = 0;
+            dep_variant = dep_default();
             return CONAN_OK;
         }
         if (mode == CONAN_DEPOSIT_LAGRANGIAN) {
@@ -515,6 +516,14 @@ template <typename T, int R> struct PM : PMBase {
         if (!mode) return set_error(CONAN_ERR_ARG, "null mode");
         *mode = lag_on() ? CONAN_DEPOSIT_LAGRANGIAN : CONAN_DEPOSIT_SORTED;
         return CONAN_OK;
+    }
+
+    // The sorted deposit's tile shape before any autotuning: the largest that
+    // gives every SM a tile, else the small one.
+    int dep_default() const {
+        typedef DepTile<R, 0> D;
+        const size_t tiles = mf.cells / ((size_t)D::TX * D::TY * D::TZ);
+        return tiles < 148 && dep_fits<DEP_SMALL>() ? DEP_SMALL : 0;
     }
 
     // Tiled deposit with tile variant V; returns 1 when V does not fit the
@@ -543,12 +552,7 @@ template <typename T, int R> struct PM : PMBase {
     int deposit() {
         if (lag_on()) return deposit_lag();
         if (!ranks_pending) CONAN_TRY(rank_pass());
-        size_t nb = (mf.cells + SCAN_CHUNK - 1) / SCAN_CHUNK;
-        CONAN_TIMED(prof, "scan", st,
-                    (k_scan_partial<<<(unsigned)nb, SCAN_T, 0, st>>>(count, mf.cells, bsum)));
-        CONAN_TIMED(prof, "scan", st, (k_scan_blocks<<<1, 1024, 0, st>>>(bsum, (int)nb)));
-        CONAN_TIMED(prof, "scan", st,
-                    (k_scan_final<<<(unsigned)nb, SCAN_T, 0, st>>>(count, mf.cells, bsum, off)));
+        CONAN_TIMED(prof, "scan", st, scan_exclusive(count, mf.cells, bsum, off, st));
         ranks_pending = false;
         CONAN_TIMED(prof, "scatter", st,
                     (k_scatter<T, R><<<grid_p(), 256, 0, st>>>(P, mf, off, rank, pay, nullptr)));
@@ -556,6 +560,7 @@ template <typename T, int R> struct PM : PMBase {
         int rc = 1;  // 1: the variant does not fit this mesh
         if (dep_variant == 1) rc = deposit_tiles<1>(scale);
         if (dep_variant == 2) rc = deposit_tiles<2>(scale);
+        if (dep_variant == DEP_SMALL) rc = deposit_tiles<DEP_SMALL>(scale);
         if (rc == 1) rc = deposit_tiles<0>(scale);
         if (rc > 1) return rc;
         if (rc == 1) {
@@ -955,6 +960,7 @@ template <typename T, int R> struct PM : PMBase {
         if (dep_fits<0>()) cands.push_back({0, 0, "sorted 32x8x8 / 256 threads"});
         if (dep_fits<1>()) cands.push_back({0, 1, "sorted 32x4x8 / 128 threads"});
         if (dep_fits<2>()) cands.push_back({0, 2, "sorted 32x16x8 / 512 threads"});
+        if (dep_fits<DEP_SMALL>()) cands.push_back({0, DEP_SMALL, "sorted, tiles of 256 cells / 256 threads"});
         if (sizeof(T) == 4 && lacc) {
             const char *tile[3] = {"", "", ""};
             if (R == 3) tile[0] = "32x8x8", tile[1] = "16x8x8", tile[2] = "8x8x8";

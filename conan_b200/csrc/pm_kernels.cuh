@@ -275,8 +275,15 @@ __device__ inline unsigned long long quant_w(double w) {
 // Tile shape of the deposit for dimension R: TX x TY x TZ output cells.
 // Variant V (0 = default) of the tile shape; the autotuner picks one per
 // mesh size.
-constexpr int DEP_VARIANTS = 3;
+// Variant DEP_SMALL has tiles of 256 cells and one particle or so per thread:
+// the default where the larger tiles are fewer than the SMs, since a tile's
+// time is its threads' chain of particles (2D FP64, 256^2: 64 tiles of 32 x 32
+// 14.1 us, 256 of 16 x 16 7.1).
+constexpr int DEP_VARIANTS = 4, DEP_SMALL = 3;
 template <int R, int V = 0> struct DepTile;
+template <> struct DepTile<3, 3> { static constexpr int TX = 8, TY = 8, TZ = 4, THREADS = 256; };
+template <> struct DepTile<2, 3> { static constexpr int TX = 16, TY = 16, TZ = 1, THREADS = 256; };
+template <> struct DepTile<1, 3> { static constexpr int TX = 256, TY = 1, TZ = 1, THREADS = 256; };
 template <> struct DepTile<3, 0> { static constexpr int TX = 32, TY = 8, TZ = 8, THREADS = 256; };
 template <> struct DepTile<3, 1> { static constexpr int TX = 32, TY = 4, TZ = 8, THREADS = 128; };
 template <> struct DepTile<3, 2> { static constexpr int TX = 32, TY = 16, TZ = 8, THREADS = 512; };

@@ -128,9 +128,7 @@ inline int radix_sort_pairs(uint64_t *k[2], uint32_t *v[2], size_t n, int bits, 
     int cur = 0;
     for (int shift = 0; shift < bits; shift += 8) {
         k_rs_hist<<<(unsigned)tiles, RS_T, 0, s>>>(k[cur], n, shift, bh, (unsigned)tiles);
-        k_scan_partial<<<(unsigned)nb, SCAN_T, 0, s>>>(bh, m, bsum);
-        k_scan_blocks<<<1, 1024, 0, s>>>(bsum, (int)nb);
-        k_scan_final<<<(unsigned)nb, SCAN_T, 0, s>>>(bh, m, bsum, boff);
+        scan_exclusive(bh, m, bsum, boff, s);
         k_rs_scatter<<<(unsigned)tiles, RS_T, RS_SMEM, s>>>(k[cur], v[cur], n, shift, boff, (unsigned)tiles,
                                                             k[cur ^ 1], v[cur ^ 1]);
         cur ^= 1;

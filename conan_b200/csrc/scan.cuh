@@ -1,5 +1,5 @@
-// scan.cuh -- exclusive prefix sum of a uint32 array in three launches
-// (block partial sums, a one-block scan of those, block-local scans), used
+// scan.cuh -- exclusive prefix sum of a uint32 array: block partial sums, a
+// one-block scan of those (large arrays), block-local scans. Used
 // for the cell offsets of the counting sorts (deposit, friends-of-friends)
 // and the group numbering of friends-of-friends.
 #pragma once
@@ -64,9 +64,18 @@ static __global__ void __launch_bounds__(1024) k_scan_blocks(uint32_t *bsum, int
 }
 
 // Exclusive offsets of every cell (off[n] = total) and counts reset to 0.
+// raw: bsum holds the block sums themselves (of at most SCAN_T blocks), which
+// each block adds up to its own; else their exclusive prefix.
 static __global__ void __launch_bounds__(SCAN_T) k_scan_final(uint32_t *__restrict__ count, size_t n,
                                                        const uint32_t *__restrict__ bsum,
-                                                       uint32_t *__restrict__ off) {
+                                                       uint32_t *__restrict__ off, bool raw) {
+    __shared__ uint32_t before;
+    if (raw) {
+        const uint32_t b = block_sum<uint32_t>(threadIdx.x < blockIdx.x ? bsum[threadIdx.x] : 0u);
+        if (threadIdx.x == 0) before = b;
+    } else if (threadIdx.x == 0) {
+        before = bsum[blockIdx.x];
+    }
     __shared__ uint32_t wsum[SCAN_T / 32];
     size_t base = (size_t)blockIdx.x * SCAN_CHUNK + (size_t)threadIdx.x * SCAN_V;
     uint32_t v[SCAN_V];
@@ -102,7 +111,7 @@ static __global__ void __launch_bounds__(SCAN_T) k_scan_final(uint32_t *__restri
     __syncthreads();
     uint32_t wpre = 0;
     for (int j = 0; j < w; ++j) wpre += wsum[j];
-    uint32_t run = bsum[blockIdx.x] + wpre + inc - s;
+    uint32_t run = before + wpre + inc - s;
     if (full) {
         uint4 *o = reinterpret_cast<uint4 *>(off + base);
 #pragma unroll
@@ -121,6 +130,19 @@ static __global__ void __launch_bounds__(SCAN_T) k_scan_final(uint32_t *__restri
         }
     }
     if (base < n && base + SCAN_V >= n) off[n] = run;
+}
+
+// off = exclusive prefix of count (off[n] = total), count = 0. bsum: one value
+// per SCAN_CHUNK counts. Up to SCAN_T blocks (1 M counts) the last launch adds
+// the block sums before its own itself; beyond, the one-block scan runs in
+// between. (65536 counts: 6.7 us in three launches, 5.1 in two; one cluster of
+// eight CTAs that exchanges its sums through distributed shared memory 9.2.)
+inline void scan_exclusive(uint32_t *count, size_t n, uint32_t *bsum, uint32_t *off, cudaStream_t s) {
+    const size_t nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    const bool raw = nb <= (size_t)SCAN_T;
+    k_scan_partial<<<(unsigned)nb, SCAN_T, 0, s>>>(count, n, bsum);
+    if (!raw) k_scan_blocks<<<1, 1024, 0, s>>>(bsum, (int)nb);
+    k_scan_final<<<(unsigned)nb, SCAN_T, 0, s>>>(count, n, bsum, off, raw);
 }
 
 }  // namespace conan
