@@ -124,7 +124,7 @@ template <typename T, int R> struct PM : PMBase {
 
     ~PM() override {
         if (st) cudaStreamSynchronize(st);
-        if (gexec) cudaGraphExecDestroy(gexec);
+        for (auto &g : pieces) cudaGraphExecDestroy(g.exec);
         fft.destroy();
         fft2.destroy();
         for (void *p : allocs) cudaFree(p);
@@ -1160,61 +1160,97 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
-    // Steps [i0, i1) of a leapfrog run starting at a(i0) = a; the first
-    // drift is separate, every later drift is fused into the previous kick.
-    int steps(double &a, double da, unsigned i0, unsigned i1) {
-        CONAN_TRY(gkd(false, 0, true, coef_drift(a, da), true));
-        a_pos = a;
+    // Steps [i0, i1) of a leapfrog run starting at a(i0) = a; the first drift
+    // (left out unless `first`) is separate, every later drift is fused into
+    // the previous kick, the last one too unless `last`.
+    int steps(double &a, double da, unsigned i0, unsigned i1, bool first = true, bool last = true) {
+        if (first) {
+            CONAN_TRY(gkd(false, 0, true, coef_drift(a, da), true));
+            a_pos = a;
+        }
         for (unsigned i = i0; i < i1; ++i) {
             double am = a + da / 2;
             CONAN_TRY(deposit_poisson(am));
-            bool last = i + 1 == i1;
+            const bool end = last && i + 1 == i1;
             double an = a + da;
-            CONAN_TRY(gkd(true, coef_kick(am, da), !last, last ? 0 : coef_drift(an, da), !last));
+            CONAN_TRY(gkd(true, coef_kick(am, da), !end, end ? 0 : coef_drift(an, da), !end));
             a_mom = am;
             a = an;
-            if (!last) a_pos = a;
+            if (!end) a_pos = a;
         }
         return CONAN_OK;
     }
 
-    // The instantiated graph of the last run segment. A later segment of the
-    // same shape (the same launches with other scale-factor coefficients)
-    // updates it in place instead of instantiating a new one.
-    cudaGraphExec_t gexec = nullptr;
+    // A run segment is captured and launched as graphs of a few steps each, so
+    // that the GPU works on one while the host captures the next (capturing
+    // 100 steps of eleven launches first took the GPU's idle millisecond of a
+    // 4.1 ms run). The instantiated graphs are kept by their shape (a piece of
+    // the same shape holds the same launches with other scale-factor
+    // coefficients, which an update in place exchanges; launches under way
+    // keep theirs).
+    static constexpr unsigned PIECE = 4;
+    struct Piece {
+        unsigned n;
+        bool first, last;
+        cudaGraphExec_t exec;
+    };
+    std::vector<Piece> pieces;
 
-    // Steps [i0, i1) captured into a CUDA graph and launched; returns after
-    // the graph has run.
-    int graph_segment(double &a, double da, unsigned i0, unsigned i1) {
+    int graph_piece(double &a, double da, unsigned i0, unsigned i1, bool first, bool last) {
         cudaGraph_t g = nullptr;
         CONAN_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        int rc = steps(a, da, i0, i1);
+        int rc = steps(a, da, i0, i1, first, last);
         cudaError_t ce = cudaStreamEndCapture(st, &g);
         if (rc != CONAN_OK) {
             if (g) cudaGraphDestroy(g);
             return rc;
         }
         if (ce != cudaSuccess) return set_error(CONAN_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
-        bool updated = false;
-        if (gexec) {
+        Piece *p = nullptr;
+        for (auto &q : pieces)
+            if (q.n == i1 - i0 && q.first == first && q.last == last) p = &q;
+        cudaError_t ie = cudaSuccess;
+        if (p) {
             cudaGraphExecUpdateResultInfo info{};
-            if (cudaGraphExecUpdate(gexec, g, &info) == cudaSuccess) {
-                updated = true;
-            } else {  // another shape: instantiate anew
+            if (cudaGraphExecUpdate(p->exec, g, &info) != cudaSuccess) {  // other launches: instantiate anew
                 cudaGetLastError();
-                cudaGraphExecDestroy(gexec);
-                gexec = nullptr;
+                cudaGraphExec_t fresh = nullptr;
+                ie = cudaGraphInstantiate(&fresh, g, 0);
+                if (ie == cudaSuccess) {
+                    cudaGraphExecDestroy(p->exec);
+                    p->exec = fresh;
+                }
+            }
+        } else {
+            if (pieces.size() >= 8) {  // bounded: the oldest shape goes
+                cudaGraphExecDestroy(pieces.front().exec);
+                pieces.erase(pieces.begin());
+            }
+            cudaGraphExec_t fresh = nullptr;
+            ie = cudaGraphInstantiate(&fresh, g, 0);
+            if (ie == cudaSuccess) {
+                pieces.push_back({i1 - i0, first, last, fresh});
+                p = &pieces.back();
             }
         }
-        cudaError_t ie = updated ? cudaSuccess : cudaGraphInstantiate(&gexec, g, 0);
         cudaGraphDestroy(g);
-        if (ie != cudaSuccess) {
-            gexec = nullptr;
-            return set_error(CONAN_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ie));
-        }
-        cudaError_t le = cudaGraphLaunch(gexec, st);
-        cudaError_t se = cudaStreamSynchronize(st);
+        if (ie != cudaSuccess) return set_error(CONAN_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ie));
+        cudaError_t le = cudaGraphLaunch(p->exec, st);
         if (le != cudaSuccess) return set_error(CONAN_ERR_CUDA, "graph launch failed: %s", cudaGetErrorString(le));
+        return CONAN_OK;
+    }
+
+    // Steps [i0, i1) as graphs; returns after they have run.
+    int graph_segment(double &a, double da, unsigned i0, unsigned i1) {
+        int rc = CONAN_OK;
+        for (unsigned i = i0; i < i1 && rc == CONAN_OK;) {
+            unsigned e = std::min(i1, i + PIECE);
+            if (i1 - e < PIECE / 2) e = i1;  // no short last piece
+            rc = graph_piece(a, da, i, e, i == i0, e == i1);
+            i = e;
+        }
+        cudaError_t se = cudaStreamSynchronize(st);
+        if (rc != CONAN_OK) return rc;
         if (se != cudaSuccess) return set_error(CONAN_ERR_CUDA, "graph execution failed: %s", cudaGetErrorString(se));
         return CONAN_OK;
     }
