@@ -70,6 +70,7 @@ SIGNATURES = {
     "conan_ic_generate": (C.c_int, [C.POINTER(ICParams), _dp, _dp]),
     "conan_ic_potential": (C.c_int, [C.POINTER(ICParams), _dp]),
     "conan_ic_displacement": (C.c_int, [C.POINTER(ICParams), _dp, _dp]),
+    "conan_release_caches": (C.c_int, []),
     "conan_cic": (C.c_int, [C.POINTER(CicParams), _dp, _dp]),
     "conan_fof": (C.c_int, [C.POINTER(FofParams), _dp, C.c_void_p, C.POINTER(C.c_ulonglong)]),
     "conan_fof_create": (C.c_void_p, [C.POINTER(FofParams)]),

@@ -10,6 +10,7 @@
 // OpenMP critical section, in thread order).
 #include <cmath>
 
+#include "hostio.cuh"
 #include "pm.cuh"
 
 namespace conan {
@@ -146,16 +147,16 @@ int cic_run(const conan_cic_params &p, const double *Xh, double *rho_h) {
         return rc == CONAN_OK;
     };
     if (fail(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream") &&
-        fail(cudaMalloc(&X, np * R * sizeof(double)), "cudaMalloc") &&
-        fail(cudaMalloc(&acc, nc * sizeof(unsigned long long)), "cudaMalloc") &&
-        fail(cudaMalloc(&rho, nc * sizeof(double)), "cudaMalloc") &&
-        fail(cudaMemcpyAsync(X, Xh, np * R * sizeof(double), cudaMemcpyHostToDevice, st), "copy") &&
-        fail(cudaMemsetAsync(acc, 0, nc * sizeof(unsigned long long), st), "memset")) {
+        fail(pool_alloc((void **)&X, np * R * sizeof(double), st), "cudaMalloc") &&
+        fail(pool_alloc((void **)&acc, nc * sizeof(unsigned long long), st), "cudaMalloc") &&
+        fail(pool_alloc((void **)&rho, nc * sizeof(double), st), "cudaMalloc") &&
+        fail(cudaMemsetAsync(acc, 0, nc * sizeof(unsigned long long), st), "memset") &&
+        (rc = copy_to_device(X, Xh, np * R * sizeof(double), st)) == CONAN_OK) {
         double mass = 1.0;
         if (s == 1) {
             k_cic_particles<R><<<(unsigned)((np + 255) / 256), 256, 0, st>>>(X, np, m, acc);
             fail(cudaGetLastError(), "k_cic_particles");
-        } else if (fail(cudaMalloc(&D, np * R * sizeof(double)), "cudaMalloc")) {
+        } else if (fail(pool_alloc((void **)&D, np * R * sizeof(double), st), "cudaMalloc")) {
             const int ns = N * s;
             const size_t nsub = (size_t)1 << (R * ilog2(ns));
             k_cic_displacement<R><<<(unsigned)((np + 255) / 256), 256, 0, st>>>(X, D, N, ilog2(N), p.size / N);
@@ -169,15 +170,14 @@ int cic_run(const conan_cic_params &p, const double *Xh, double *rho_h) {
             k_cic_finish<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(acc, rho, nc, mass / CIC_UNIT);
             fail(cudaGetLastError(), "k_cic_finish");
         }
-        if (rc == CONAN_OK) fail(cudaMemcpyAsync(rho_h, rho, nc * sizeof(double), cudaMemcpyDeviceToHost, st), "copy");
+        if (rc == CONAN_OK) rc = copy_to_host(rho_h, rho, nc * sizeof(double), st);
         if (rc == CONAN_OK) fail(cudaStreamSynchronize(st), "run");
     }
-    if (st) cudaStreamSynchronize(st);
-    cudaFree(X);
-    cudaFree(D);
-    cudaFree(acc);
-    cudaFree(rho);
-    if (st) cudaStreamDestroy(st);
+    if (st) {
+        for (void *q : {(void *)X, (void *)D, (void *)acc, (void *)rho}) pool_free(q, st);
+        cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
+    }
     return rc;
 }
 

@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "hostio.cuh"
 #include "pm.cuh"
 #include "radix.cuh"
 #include "scan.cuh"
@@ -651,9 +652,9 @@ struct FofEngine {
     }
 
     int run_host(const double *Xh, unsigned long long *tg_h, uint64_t *ngroups) {
-        CONAN_CUDA(cudaMemcpyAsync(X, Xh, n * R * sizeof(double), cudaMemcpyHostToDevice, st));
+        CONAN_TRY(copy_to_device(X, Xh, n * R * sizeof(double), st));
         CONAN_TRY(run_device(X, tags, st, ngroups));
-        CONAN_CUDA(cudaMemcpyAsync(tg_h, tags, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        CONAN_TRY(copy_to_host(tg_h, tags, n * sizeof(unsigned long long), st));
         CONAN_CUDA(cudaStreamSynchronize(st));
         return CONAN_OK;
     }

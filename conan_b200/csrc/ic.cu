@@ -6,7 +6,7 @@
 #include <cmath>
 #include <vector>
 
-#include "fft.cuh"
+#include "hostio.cuh"
 #include "ic.cuh"
 #include "pm.cuh"
 
@@ -307,7 +307,7 @@ int check_ic_params(const conan_ic_params *p) {
 // Scoped device buffers and plan for one ic call.
 template <typename T> struct ICWork {
     typedef typename Cplx<T>::type CT;
-    Mesh m;
+    Mesh m{};
     T *mesh = nullptr;
     CT *spec = nullptr, *spec2 = nullptr;
     double *xfer = nullptr, *part = nullptr;
@@ -315,33 +315,35 @@ template <typename T> struct ICWork {
     FFTPair fft;
     cudaStream_t st = nullptr;
     ~ICWork() {
-        if (st) cudaStreamSynchronize(st);
-        fft.destroy();
-        cudaFree(mesh);
-        cudaFree(spec);
-        cudaFree(spec2);
-        cudaFree(xfer);
-        cudaFree(part);
-        cudaFree(work);
-        if (st) cudaStreamDestroy(st);
+        if (!st) return;
+        for (void *p : {(void *)mesh, (void *)spec, (void *)spec2, (void *)xfer, (void *)part, work}) pool_free(p, st);
+        cudaStreamSynchronize(st);
+        plan_return(m, sizeof(T) == 8, &fft);
+        cudaStreamDestroy(st);
+    }
+    template <typename U> int alloc(U **p, size_t n) {
+        void *q = nullptr;
+        CONAN_CUDA(pool_alloc(&q, n * sizeof(U), st));
+        *p = (U *)q;
+        return CONAN_OK;
     }
     int setup(const conan_ic_params &p, bool need_spec2) {
         m = make_mesh(p.dim, 1 << p.mbits);
         CONAN_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        CONAN_CUDA(cudaMalloc(&mesh, m.cells * sizeof(T)));
-        CONAN_CUDA(cudaMalloc(&spec, m.spec * sizeof(CT)));
-        if (need_spec2) CONAN_CUDA(cudaMalloc(&spec2, m.spec * sizeof(CT)));
-        CONAN_CUDA(cudaMalloc(&xfer, m.cells * sizeof(double) * (need_spec2 ? p.dim : 1)));
-        CONAN_CUDA(cudaMalloc(&part, ic_scratch(m) * sizeof(double)));
-        CONAN_TRY(fft.create(m, sizeof(T) == 8, 1));
-        CONAN_CUDA(cudaMalloc(&work, fft.work_bytes ? fft.work_bytes : 16));
+        CONAN_TRY(alloc(&mesh, m.cells));
+        CONAN_TRY(alloc(&spec, m.spec));
+        if (need_spec2) CONAN_TRY(alloc(&spec2, m.spec));
+        CONAN_TRY(alloc(&xfer, m.cells * (need_spec2 ? p.dim : 1)));
+        CONAN_TRY(alloc(&part, ic_scratch(m)));
+        CONAN_TRY(plan_take(m, sizeof(T) == 8, &fft));
+        CONAN_TRY(alloc((char **)&work, fft.work_bytes ? fft.work_bytes : 16));
         CONAN_TRY(fft.bind(work, st));
         return CONAN_OK;
     }
     unsigned gc() const { return (unsigned)((m.cells + 255) / 256); }
     unsigned gs() const { return (unsigned)((m.spec + 255) / 256); }
     int upload(const double *h) {
-        CONAN_CUDA(cudaMemcpyAsync(xfer, h, m.cells * sizeof(double), cudaMemcpyHostToDevice, st));
+        CONAN_TRY(copy_to_device(xfer, h, m.cells * sizeof(double), st));
         k_convert<double, T><<<gc(), 256, 0, st>>>(xfer, mesh, m.cells, 1.0, 0.0);
         CONAN_LAUNCHED();
         return CONAN_OK;
@@ -349,7 +351,7 @@ template <typename T> struct ICWork {
     int download(double *h) {
         k_convert<T, double><<<gc(), 256, 0, st>>>(mesh, xfer, m.cells, 1.0, 0.0);
         CONAN_LAUNCHED();
-        CONAN_CUDA(cudaMemcpyAsync(h, xfer, m.cells * sizeof(double), cudaMemcpyDeviceToHost, st));
+        CONAN_TRY(copy_to_host(h, xfer, m.cells * sizeof(double), st));
         CONAN_CUDA(cudaStreamSynchronize(st));
         return CONAN_OK;
     }
@@ -547,7 +549,7 @@ template <typename T> int ic_displacement(const conan_ic_params &p, const double
         k_interleave<T><<<w.gc(), 256, 0, w.st>>>(w.mesh, w.xfer, w.m.cells, p.dim, a);
         CONAN_LAUNCHED();
     }
-    CONAN_CUDA(cudaMemcpyAsync(psi, w.xfer, w.m.cells * p.dim * sizeof(double), cudaMemcpyDeviceToHost, w.st));
+    CONAN_TRY(copy_to_host(psi, w.xfer, w.m.cells * p.dim * sizeof(double), w.st));
     CONAN_CUDA(cudaStreamSynchronize(w.st));
     return CONAN_OK;
 }
@@ -567,7 +569,7 @@ int conan_ic_noise(const conan_ic_params *p, double *noise_out) {
     size_t pairs = (w.m.cells + 1) / 2;
     k_noise_philox_f64<<<(unsigned)((pairs + 255) / 256), 256, 0, w.st>>>(w.xfer, w.m.cells, p->seed);
     CONAN_LAUNCHED();
-    CONAN_CUDA(cudaMemcpyAsync(noise_out, w.xfer, w.m.cells * sizeof(double), cudaMemcpyDeviceToHost, w.st));
+    CONAN_TRY(copy_to_host(noise_out, w.xfer, w.m.cells * sizeof(double), w.st));
     CONAN_CUDA(cudaStreamSynchronize(w.st));
     return CONAN_OK;
 }

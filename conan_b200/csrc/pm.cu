@@ -14,6 +14,7 @@
 #define PLANE_CLEAR 1
 #endif
 #include "fft_z.cuh"
+#include "hostio.cuh"
 #include "ic.cuh"
 #include "pm.cuh"
 
@@ -136,6 +137,11 @@ template <typename T, int R> struct PM : PMBase {
         size_t b = n * sizeof(U);
         if (b == 0) b = 16;
         cudaError_t e = cudaMalloc(&q, b);
+        if (e == cudaErrorMemoryAllocation) {  // what the handle-less calls keep idle may be enough
+            cudaGetLastError();
+            release_caches();
+            e = cudaMalloc(&q, b);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             return set_error(CONAN_ERR_ALLOC, "cudaMalloc of %zu bytes failed: %s", b, cudaGetErrorString(e));
@@ -234,12 +240,8 @@ template <typename T, int R> struct PM : PMBase {
             CONAN_TIMED(prof, "export", st,
                         (k_export<T, R><<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(
                             v, res_f, i0, cnt, X ? stage[0] : nullptr, Pm ? stage[1] : nullptr)));
-            if (X)
-                CONAN_CUDA(cudaMemcpyAsync(X + i0 * R, stage[0], cnt * R * sizeof(double), cudaMemcpyDeviceToHost,
-                                           st));
-            if (Pm)
-                CONAN_CUDA(cudaMemcpyAsync(Pm + i0 * R, stage[1], cnt * R * sizeof(double), cudaMemcpyDeviceToHost,
-                                           st));
+            if (X) CONAN_TRY(copy_to_host(X + i0 * R, stage[0], cnt * R * sizeof(double), st));
+            if (Pm) CONAN_TRY(copy_to_host(Pm + i0 * R, stage[1], cnt * R * sizeof(double), st));
         }
         CONAN_CUDA(cudaStreamSynchronize(st));
         return CONAN_OK;
@@ -250,7 +252,7 @@ template <typename T, int R> struct PM : PMBase {
     int upload_mesh(const double *in, T *out, size_t n) {
         for (size_t c0 = 0, b = 0; c0 < n; c0 += stage_n, b ^= 1) {
             const size_t cnt = std::min(stage_n, n - c0);
-            CONAN_CUDA(cudaMemcpyAsync(stage[b], in + c0, cnt * sizeof(double), cudaMemcpyHostToDevice, st));
+            CONAN_TRY(copy_to_device(stage[b], in + c0, cnt * sizeof(double), st));
             CONAN_TIMED(prof, "convert", st,
                         (k_convert<double, T><<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(stage[b], out + c0, cnt,
                                                                                           1.0, 0.0)));
@@ -1302,8 +1304,8 @@ template <typename T, int R> struct PM : PMBase {
         const size_t cp = stage_particles();
         for (size_t i0 = 0; i0 < np; i0 += cp) {
             const size_t cnt = std::min(cp, np - i0);
-            CONAN_CUDA(cudaMemcpyAsync(stage[0], X + i0 * R, cnt * R * sizeof(double), cudaMemcpyHostToDevice, st));
-            CONAN_CUDA(cudaMemcpyAsync(stage[1], Pm + i0 * R, cnt * R * sizeof(double), cudaMemcpyHostToDevice, st));
+            CONAN_TRY(copy_to_device(stage[0], X + i0 * R, cnt * R * sizeof(double), st));
+            CONAN_TRY(copy_to_device(stage[1], Pm + i0 * R, cnt * R * sizeof(double), st));
             CONAN_TIMED(prof, "import", st,
                         (k_import<T, R><<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(P, res_f, i0, cnt, stage[0],
                                                                                        stage[1])));
@@ -1321,7 +1323,7 @@ template <typename T, int R> struct PM : PMBase {
             CONAN_TIMED(prof, "convert", st,
                         (k_convert<T, double><<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(mesh + c0, stage[b], cnt,
                                                                                           1.0, 0.0)));
-            CONAN_CUDA(cudaMemcpyAsync(out + c0, stage[b], cnt * sizeof(double), cudaMemcpyDeviceToHost, st));
+            CONAN_TRY(copy_to_host(out + c0, stage[b], cnt * sizeof(double), st));
         }
         CONAN_CUDA(cudaStreamSynchronize(st));
         return check_err();

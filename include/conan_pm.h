@@ -103,6 +103,12 @@ int conan_ic_potential(const conan_ic_params *p, double *inout);
  * without the file write: psi_out receives N^dim x dim doubles (AoS). */
 int conan_ic_displacement(const conan_ic_params *p, const double *potential, double *psi_out);
 
+/* Calls that take host arrays keep a bounded cache for the next ones: per
+ * device at most 16 MiB of page-locked staging memory and 512 MiB of device
+ * memory, and four pairs of FFT plans. This gives all of it back (what calls
+ * under way on other threads hold stays theirs). No reference counterpart. */
+int conan_release_caches(void);
+
 /* ----------------------------------------------------------------- cic -- */
 
 /* Options of the `cic` tool, src/cic/main.cc:17-32, with the snapshot's box. */
