@@ -193,7 +193,8 @@ template <typename T, int R> struct PM : PMBase {
         CONAN_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
         CONAN_CUDA(cudaMemsetAsync(count, 0, mf.cells * sizeof(uint32_t), st));
         dep_variant = dep_default();
-        bool lag = sizeof(T) == 4 && (lag_try<0>() || lag_try<1>() || lag_try<2>());
+        bool lag = sizeof(T) == 4 && ((lag_small<R>(np) && lag_try<LAG_SMALL>()) || lag_try<0>() || lag_try<1>() ||
+                                  lag_try<2>());
         // On fine meshes (f >= 2) a window that fits shared memory only fits
         // a small tile and holds many cells per particle, each of which gets
         // about one corner: clearing and flushing it costs more than the
@@ -280,7 +281,7 @@ template <typename T, int R> struct PM : PMBase {
         return (double)LagTile<R, V>::LX * LagTile<R, V>::LY * LagTile<R, V>::LZ;
     }
     double lag_particles() const {
-        return lag_v == 0 ? lag_tile_particles<0>() : lag_v == 1 ? lag_tile_particles<1>() : lag_tile_particles<2>();
+        return lag_v == 0 ? lag_tile_particles<0>() : lag_v == 1 ? lag_tile_particles<1>() : lag_v == 2 ? lag_tile_particles<2>() : lag_tile_particles<3>();
     }
 
     // direct: a window of two cells per axis, so that (nearly) every corner
@@ -335,6 +336,7 @@ template <typename T, int R> struct PM : PMBase {
             if (lag_v == 0) return tma_setup_v<0>();
             if (lag_v == 1) return tma_setup_v<1>();
             if (lag_v == 2) return tma_setup_v<2>();
+            if (lag_v == 3) return tma_setup_v<3>();
         }
         return CONAN_OK;
     }
@@ -473,9 +475,16 @@ template <typename T, int R> struct PM : PMBase {
     // mesh (unless the fused gather kernel did it already).
     int lag_accumulate() {
         if (!lag_ready) {
-            if (lag_v == 0) CONAN_TRY(launch_lag<0>());
+            if (tma_ok && !pers_ok) {  // the staged tiles, neither kick nor drift
+                const GKD c{0, 0, 0, 0, 0, 0};
+                if (lag_v == 0) CONAN_TRY(launch_gkd_lag<0>(c, "deposit"));
+                else if (lag_v == 1) CONAN_TRY(launch_gkd_lag<1>(c, "deposit"));
+                else if (lag_v == 2) CONAN_TRY(launch_gkd_lag<2>(c, "deposit"));
+                else CONAN_TRY(launch_gkd_lag<3>(c, "deposit"));
+            } else if (lag_v == 0) CONAN_TRY(launch_lag<0>());
             else if (lag_v == 1) CONAN_TRY(launch_lag<1>());
-            else CONAN_TRY(launch_lag<2>());
+            else if (lag_v == 2) CONAN_TRY(launch_lag<2>());
+            else CONAN_TRY(launch_lag<3>());
         }
         lag_ready = false;
         return CONAN_OK;
@@ -888,7 +897,8 @@ template <typename T, int R> struct PM : PMBase {
         return mf.n >= D::TX && mf.n >= D::TY && mf.n >= D::TZ;
     }
     bool lag_set(int v, bool direct) {
-        return v == 0 ? lag_try<0>(direct) : v == 1 ? lag_try<1>(direct) : lag_try<2>(direct);
+        return v == 0 ? lag_try<0>(direct) : v == 1 ? lag_try<1>(direct) : v == 2 ? lag_try<2>(direct)
+                                                                                 : lag_try<LAG_SMALL>(direct);
     }
     int dep_apply(const DepCand &c) {
         CONAN_TRY(drop_lag_deposit());
@@ -964,11 +974,11 @@ template <typename T, int R> struct PM : PMBase {
         if (dep_fits<2>()) cands.push_back({0, 2, "sorted 32x16x8 / 512 threads"});
         if (dep_fits<DEP_SMALL>()) cands.push_back({0, DEP_SMALL, "sorted, tiles of 256 cells / 256 threads"});
         if (sizeof(T) == 4 && lacc) {
-            const char *tile[3] = {"", "", ""};
-            if (R == 3) tile[0] = "32x8x8", tile[1] = "16x8x8", tile[2] = "8x8x8";
-            if (R == 2) tile[0] = "64x32", tile[1] = "32x16", tile[2] = "16x16";
+            const char *tile[4] = {"", "", "", ""};
+            if (R == 3) tile[0] = "32x8x8", tile[1] = "16x8x8", tile[2] = "8x8x8", tile[3] = "16x8x4";
+            if (R == 2) tile[0] = "64x32", tile[1] = "32x16", tile[2] = "16x16", tile[3] = "16x16 / 256 threads";
             if (R == 1) tile[0] = "2048", tile[1] = "512", tile[2] = "128";
-            for (int v = 0; v < 3; ++v)
+            for (int v = 0; v < (lag_small<R>(np) ? 4 : 3); ++v)
                 if (lag_set(v, false)) cands.push_back({1, v, std::string("lagrangian window, tile ") + tile[v]});
             if (R == 3)
                 for (int v = 0; v < 2; ++v)
@@ -1103,7 +1113,8 @@ template <typename T, int R> struct PM : PMBase {
             const char *fname = kick ? "gather_kick_drift_deposit" : "drift_deposit";
             if (lag_v == 0) CONAN_TRY(launch_gkd_lag<0>(c, fname));
             else if (lag_v == 1) CONAN_TRY(launch_gkd_lag<1>(c, fname));
-            else CONAN_TRY(launch_gkd_lag<2>(c, fname));
+            else if (lag_v == 2) CONAN_TRY(launch_gkd_lag<2>(c, fname));
+            else CONAN_TRY(launch_gkd_lag<3>(c, fname));
             lag_ready = true;
             return CONAN_OK;
         }
@@ -1113,7 +1124,8 @@ template <typename T, int R> struct PM : PMBase {
             c.deposit = 0;
             if (lag_v == 0) CONAN_TRY(launch_gkd_lag<0>(c, name));
             else if (lag_v == 1) CONAN_TRY(launch_gkd_lag<1>(c, name));
-            else CONAN_TRY(launch_gkd_lag<2>(c, name));
+            else if (lag_v == 2) CONAN_TRY(launch_gkd_lag<2>(c, name));
+            else CONAN_TRY(launch_gkd_lag<3>(c, name));
             return CONAN_OK;
         }
         if (prm.gradient == CONAN_GRAD_SPECTRAL)

@@ -826,7 +826,7 @@ struct LagWin {
 
 // Lattice tile (LX x LY x LZ particles), threads and window margin M (cells
 // beyond the tile's own f*L cells, split over both sides) of variant V.
-constexpr int LAG_VARIANTS = 3;
+constexpr int LAG_VARIANTS = 4;
 // 32-bit planes of a window cell: 2 keeps the carry in shared memory, 1
 // sends it to the accumulator mesh (a carry needs over 2^9 particles' weight
 // in one cell of one tile: rare). A compile-time tunable; one plane leaves
@@ -846,12 +846,28 @@ template <int R, int V> struct LagTile;
 template <> struct LagTile<3, 0> { static constexpr int LX = 32, LY = 8, LZ = 8, THREADS = 512, M = 8; };
 template <> struct LagTile<3, 1> { static constexpr int LX = 16, LY = 8, LZ = 8, THREADS = 256, M = 8; };
 template <> struct LagTile<3, 2> { static constexpr int LX = 8, LY = 8, LZ = 8, THREADS = 128, M = 8; };
+// LAG_SMALL: half a tile or less per CTA and one or two particles per thread,
+// for lattices whose tiles of this shape all run at once (lag_small): there a
+// launch takes as long as one tile's chain (gather + kick + drift + deposit:
+// 32^3 9 -> 5 us, 64^3 11 -> 9; on larger lattices its windows overlap more:
+// 128^3 60 -> 64 us).
+constexpr int LAG_SMALL = 3;
+template <> struct LagTile<3, 3> { static constexpr int LX = 16, LY = 8, LZ = 4, THREADS = 256, M = 8; };
+template <> struct LagTile<2, 3> { static constexpr int LX = 16, LY = 16, LZ = 1, THREADS = 256, M = 16; };
+template <> struct LagTile<1, 3> { static constexpr int LX = 128, LY = 1, LZ = 1, THREADS = 128, M = 32; };
 template <> struct LagTile<2, 0> { static constexpr int LX = 64, LY = 32, LZ = 1, THREADS = 512, M = 16; };
 template <> struct LagTile<2, 1> { static constexpr int LX = 32, LY = 16, LZ = 1, THREADS = 128, M = 16; };
 template <> struct LagTile<2, 2> { static constexpr int LX = 16, LY = 16, LZ = 1, THREADS = 64, M = 16; };
 template <> struct LagTile<1, 0> { static constexpr int LX = 2048, LY = 1, LZ = 1, THREADS = 512, M = 64; };
 template <> struct LagTile<1, 1> { static constexpr int LX = 512, LY = 1, LZ = 1, THREADS = 128, M = 64; };
 template <> struct LagTile<1, 2> { static constexpr int LX = 128, LY = 1, LZ = 1, THREADS = 32, M = 32; };
+
+// Whether the LAG_SMALL tiles of np particles are one wave: four CTAs of 256
+// threads (64 registers each) on each of 148 SMs.
+template <int R> inline bool lag_small(size_t np) {
+    typedef LagTile<R, LAG_SMALL> L;
+    return R > 1 && np <= (size_t)(4 * 148) * (L::LX * L::LY * L::LZ);
+}
 
 // The body of the Lagrangian deposit for one lattice tile. FUSED: the
 // particles are first advanced as in k_gkd (gather of the packed gradient,
@@ -940,7 +956,10 @@ __device__ __forceinline__ void gather_g4(const G4<float> *__restrict__ Gm, int 
 // the phase parity of this use of the staging buffer's barriers and the
 // window (kept clear between tiles: the flush zeroes what it reads) come
 // from the caller.
-template <int R, int LX, int LY, int LZ, int THREADS, bool FUSED, bool STAGED = false, bool PERSIST = false>
+// LATE: the accumulator may still be written by the kernel before this one
+// (programmatic dependent launch): wait for it before the first add.
+template <int R, int LX, int LY, int LZ, int THREADS, bool FUSED, bool STAGED = false, bool PERSIST = false,
+          bool LATE = false>
 __device__ __forceinline__ void lag_tile(const Parts<float> &P, const Mesh &m, const LagWin &win,
                                          unsigned long long *__restrict__ acc, const G4<float> *__restrict__ G,
                                          const GKD &gc, float *stage = nullptr,
@@ -1099,6 +1118,7 @@ __device__ __forceinline__ void lag_tile(const Parts<float> &P, const Mesh &m, c
     }
     if (threadIdx.x >= R && threadIdx.x < 3) org[3 + threadIdx.x] = 1;
     __syncthreads();
+    if constexpr (LATE) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const int o0 = org[0], o1 = R >= 2 ? org[1] : 0, o2 = R == 3 ? org[2] : 0;
     const int W0 = win.w[0], W1 = win.w[1], W2 = win.w[2], W01 = W0 * W1;
@@ -1310,7 +1330,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 #pragma unroll
         for (int j = 0; j < NPT; ++j) {
             const uint32_t b = smem_addr(bars + j);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(6u * THREADS * 4u)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b),
+                         "r"(6u * THREADS * 4u)
                          : "memory");
             // group j: the planes s NPT + j, one box (LX x LY x 1) each
 #pragma unroll
