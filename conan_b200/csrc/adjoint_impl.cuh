@@ -505,11 +505,12 @@ template <typename T, int R> struct Diff : DiffBase {
     unsigned kev() const { return prm.checkpoint_every ? prm.checkpoint_every : 1; }
     dim3 gp() const { return dim3((unsigned)((pm.np + 255) / 256)); }
 
+    // Orders the handle's stream after the caller's work. NULL is the legacy
+    // default stream (where torch enqueues unless told otherwise), which a
+    // non-blocking stream does not wait for by itself.
     int enter(void *stream) {
-        if (stream) {
-            CONAN_CUDA(cudaEventRecord(ev, (cudaStream_t)stream));
-            CONAN_CUDA(cudaStreamWaitEvent(pm.st, ev, 0));
-        }
+        CONAN_CUDA(cudaEventRecord(ev, stream ? (cudaStream_t)stream : cudaStreamLegacy));
+        CONAN_CUDA(cudaStreamWaitEvent(pm.st, ev, 0));
         return CONAN_OK;
     }
     int leave(void *stream) {

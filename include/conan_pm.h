@@ -303,7 +303,8 @@ conan_diff *conan_diff_create(const conan_diff_params *p);
 void conan_diff_destroy(conan_diff *h);
 /* Device pointers of the handle's precision (float or double):
  * noise N^dim, density_out N_f^dim. `stream` is a cudaStream_t (NULL: the
- * handle's stream); the call is ordered after prior work on it. */
+ * legacy default stream); the call is ordered after prior work on it, and
+ * later work on it after the call (with NULL the call waits for its work). */
 int conan_diff_forward(conan_diff *h, const void *noise_dev, void *density_out_dev, void *stream);
 /* Gradient of a scalar loss w.r.t. the noise given its gradient w.r.t. the
  * final density of the last forward call. */
