@@ -220,6 +220,7 @@ template <typename T, int R> struct PM : PMBase {
         }
         // CONAN_GRAD_KERNEL: cell or zm picks the gradient-mesh kernel at
         // creation (before any autotuning)
+        grad_zm = mf.cells > ((size_t)1 << 21);
         if (const char *gk = getenv("CONAN_GRAD_KERNEL")) grad_zm = !strcmp(gk, "zm");
         CONAN_TRY(alloc((char **)&work, wbytes));
         CONAN_TRY(fft.bind(work, st));
@@ -846,20 +847,20 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
-    // Packed FD4 gradient mesh of phi. (Measured at 512^3: the plain
-    // thread-per-cell kernel beats four-cells-per-thread and warp-shuffle
-    // variants, 0.64 against 0.68 and 0.83 ms.)
-    // Gradient-mesh kernel: z-marching tiles (3D, 32 cells per side and
-    // more) or one thread per cell in blocks of grad_block threads; the
-    // autotuner picks one.
-    bool grad_zm = FD_GRAD_ZM != 0;
+    // Packed FD4 gradient mesh of phi. Gradient-mesh kernel: columns marching
+    // along z (3D, 32 cells per side and more) or one thread per cell in blocks
+    // of grad_block threads. The default marches on meshes beyond 2^21 cells,
+    // whose potential and gradient leave the L2 (256^3 86 -> 70 us; 128^3 10 us
+    // either way, 64^3 2.6 against 3.4 us with a quarter of the threads); the
+    // autotuner times both.
+    bool grad_zm = false;
     int grad_block = 256;
     bool grad_zm_fits() const { return R == 3 && mf.n >= 32; }
 
     int fd_gradient(const T *phi, G4<T> *g) {
         if constexpr (R == 3) {
             if (grad_zm && grad_zm_fits()) {
-                const unsigned blocks = (unsigned)((size_t)(mf.n / 32) * (mf.n / 8) * (mf.n / FDZ_PLANES) * mf.batch);
+                const unsigned blocks = (unsigned)(mf.cells / (256 * FDZ_PLANES));
                 CONAN_TIMED(prof, "fd_grad", st, (k_fd_grad_zm<T><<<blocks, 256, 0, st>>>(phi, g, mf)));
                 return CONAN_OK;
             }
@@ -1008,7 +1009,7 @@ template <typename T, int R> struct PM : PMBase {
             struct GC { bool zm; int block; std::string name; };
             std::vector<GC> g = {{false, 128, "thread per cell, 128"}, {false, 256, "thread per cell, 256"},
                                  {false, 512, "thread per cell, 512"}};
-            if (grad_zm_fits()) g.push_back({true, 256, "z-marching 32x8 tiles"});
+            if (grad_zm_fits()) g.push_back({true, 256, "z-marching columns"});
             best = -1;
             bms = 1e30;
             for (size_t i = 0; i < g.size(); ++i) {
