@@ -605,13 +605,11 @@ template <typename T, int R> struct Diff : DiffBase {
     int adjoint_poisson(double am) {
         CONAN_TRY(neg_div(U, S, rhobar, pm.mf));
         const double gsc = pm.poisson_scale(am);
-        if constexpr (sizeof(T) == 4) {
-            if (pm.zpass) {  // the forward solve's plane transforms and z pass
-                CONAN_TRY(pm.fft2.forward(rhobar, pm.spec));
-                CONAN_TRY(pm.green_z(gsc));
-                CONAN_TRY(pm.fft2.inverse(pm.spec, rhobar));
-                return CONAN_OK;
-            }
+        if (pm.zpass) {  // the forward solve's plane transforms and z pass
+            CONAN_TRY(pm.fft2.forward(rhobar, pm.spec));
+            CONAN_TRY(pm.green_z(gsc));
+            CONAN_TRY(pm.fft2.inverse(pm.spec, rhobar));
+            return CONAN_OK;
         }
         CONAN_TRY(pm.fft.forward(rhobar, pm.spec));
         CONAN_TRY(pm.green(pm.spec, gsc));

@@ -31,21 +31,22 @@ struct FFTPair {
         work_bytes = w1 > w2 ? w1 : w2;
         return CONAN_OK;
     }
-    // 2D transforms of every z plane (3D meshes): the same half-spectrum
-    // layout as the 3D pair with z left in real space.
+    // The same half-spectrum layout with the slowest axis left in real space: 2D
+    // transforms of every z plane of 3D meshes, 1D ones of every row of 2D ones.
     int create_planes(const Mesh &m, bool is_double, int batch) {
         dbl = is_double;
         int n[2] = {m.n, m.n};
-        long long real_dist = (long long)m.n * m.n, cplx_dist = (long long)m.n * m.nh;
+        const int rank = m.R - 1;
+        long long real_dist = rank == 2 ? (long long)m.n * m.n : m.n, cplx_dist = rank == 2 ? (long long)m.n * m.nh : m.nh;
         const int planes = batch * m.n;
         size_t w1 = 0, w2 = 0;
         CONAN_CUFFT(cufftCreate(&r2c));
         CONAN_CUFFT(cufftCreate(&c2r));
         CONAN_CUFFT(cufftSetAutoAllocation(r2c, 0));
         CONAN_CUFFT(cufftSetAutoAllocation(c2r, 0));
-        CONAN_CUFFT(cufftMakePlanMany(r2c, 2, n, nullptr, 1, (int)real_dist, nullptr, 1, (int)cplx_dist,
+        CONAN_CUFFT(cufftMakePlanMany(r2c, rank, n, nullptr, 1, (int)real_dist, nullptr, 1, (int)cplx_dist,
                                       dbl ? CUFFT_D2Z : CUFFT_R2C, planes, &w1));
-        CONAN_CUFFT(cufftMakePlanMany(c2r, 2, n, nullptr, 1, (int)cplx_dist, nullptr, 1, (int)real_dist,
+        CONAN_CUFFT(cufftMakePlanMany(c2r, rank, n, nullptr, 1, (int)cplx_dist, nullptr, 1, (int)real_dist,
                                       dbl ? CUFFT_Z2D : CUFFT_C2R, planes, &w2));
         work_bytes = w1 > w2 ? w1 : w2;
         return CONAN_OK;

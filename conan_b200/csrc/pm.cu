@@ -13,6 +13,7 @@
 #ifndef PLANE_CLEAR
 #define PLANE_CLEAR 1
 #endif
+#include "fft_line64.cuh"
 #include "fft_z.cuh"
 #include "hostio.cuh"
 #include "ic.cuh"
@@ -111,8 +112,9 @@ template <typename T, int R> struct PM : PMBase {
     FFTPair fft;
     // FP32 3D FD4 meshes of 64..1024 cells per side: the Poisson solve as 2D
     // transforms of the z planes around the shared-memory z pass (fft_z.cuh)
+    // (FP64, 2D of 64..1024 and 3D of 64..512 cells per side: fft_line64.cuh)
     FFTPair fft2;
-    float2 *ztw = nullptr;  // exp(-2 pi i k / n), k < n
+    CT *ztw = nullptr;  // exp(-2 pi i k / n), k < n
     bool zpass = false;
     cudaStream_t st = nullptr;
     Profiler prof;
@@ -211,8 +213,9 @@ template <typename T, int R> struct PM : PMBase {
         }
         CONAN_TRY(fft.create(mf, sizeof(T) == 8, batch));
         size_t wbytes = fft.work_bytes;
-        if (sizeof(T) == 4 && R == 3 && p.gradient == CONAN_GRAD_FD4 && mf.n >= 64 && mf.n <= 1024) {
-            CONAN_TRY(fft2.create_planes(mf, false, batch));
+        const bool split = sizeof(T) == 4 ? R == 3 && mf.n <= 1024 : (R == 3 && mf.n <= 512) || (R == 2 && mf.n <= 1024);
+        if (split && p.gradient == CONAN_GRAD_FD4 && mf.n >= 64) {
+            CONAN_TRY(fft2.create_planes(mf, sizeof(T) == 8, batch));
             CONAN_TRY(zpass_setup());
             wbytes = std::max(wbytes, fft2.work_bytes);
             zpass = true;
@@ -594,19 +597,52 @@ template <typename T, int R> struct PM : PMBase {
     }
 
     int zpass_setup() {
-        std::vector<float2> w((size_t)mf.n);
+        std::vector<CT> w((size_t)mf.n);
         for (int k = 0; k < mf.n; ++k) {
             const double a = -2.0 * M_PI * (double)k / (double)mf.n;
-            w[k] = make_float2((float)std::cos(a), (float)std::sin(a));
+            w[k].x = (T)std::cos(a);
+            w[k].y = (T)std::sin(a);
         }
         CONAN_TRY(alloc(&ztw, (size_t)mf.n));
-        CONAN_CUDA(cudaMemcpy(ztw, w.data(), w.size() * sizeof(float2), cudaMemcpyHostToDevice));
+        CONAN_CUDA(cudaMemcpy(ztw, w.data(), w.size() * sizeof(CT), cudaMemcpyHostToDevice));
+        if constexpr (sizeof(T) == 4) {
+            switch (mf.n) {
+                case 64: return zpass_attr<64>();
+                case 128: return zpass_attr<128>();
+                case 256: return zpass_attr<256>();
+                case 512: return zpass_attr<512>();
+                default: return zpass_attr<1024>();
+            }
+        } else {
+            return line_green(0.0, true);
+        }
+    }
+    // The FP64 line pass of this mesh; attr: only set its shared-memory limit.
+    int line_green(double gs, bool attr = false) {
         switch (mf.n) {
-            case 64: return zpass_attr<64>();
-            case 128: return zpass_attr<128>();
-            case 256: return zpass_attr<256>();
-            case 512: return zpass_attr<512>();
-            default: return zpass_attr<1024>();
+            case 64: return line_green_n<64>(gs, attr);
+            case 128: return line_green_n<128>(gs, attr);
+            case 256: return line_green_n<256>(gs, attr);
+            case 512: return line_green_n<512>(gs, attr);
+            default: return line_green_n<1024>(gs, attr);
+        }
+    }
+    template <int N> int line_green_n(double gs, bool attr) {
+        if constexpr (sizeof(T) == 8 && (R == 2 || (R == 3 && N <= 512))) {
+            typedef LineT<N, R> L;
+            auto k = k_line_green64<N, R>;
+            if (attr) {
+                if (!raise_dyn_smem(k, L::SMEM))
+                    return set_error(CONAN_ERR_CUDA, "line pass: %zu bytes of shared memory refused", L::SMEM);
+                return CONAN_OK;
+            }
+            const dim3 grid((unsigned)((mf.nh + L::TX - 1) / L::TX), R == 3 ? (unsigned)mf.n : 1u, (unsigned)mf.batch);
+            CONAN_TIMED(prof, "green", st,
+                        (k<<<grid, L::THREADS, L::SMEM, st>>>(reinterpret_cast<double2 *>(spec), mf, gs,
+                                                              reinterpret_cast<const double2 *>(ztw))));
+            return CONAN_OK;
+        } else {
+            return set_error(CONAN_ERR_UNSUPPORTED, "no line pass for this mesh");
         }
     }
     // z-pass lines per CTA: 0 the default width, else TX (the autotuner's knob)
@@ -645,7 +681,8 @@ template <typename T, int R> struct PM : PMBase {
         if constexpr (ZTile<N, TX>::OK) {
             typedef ZTile<N, TX> Z;
             const dim3 grid((unsigned)((mf.nh + Z::TX - 1) / Z::TX), (unsigned)mf.n, (unsigned)mf.batch);
-            k_zpass_green<N, TX><<<grid, Z::THREADS, Z::SMEM, st>>>(reinterpret_cast<float2 *>(spec), mf, gs, ztw);
+            k_zpass_green<N, TX><<<grid, Z::THREADS, Z::SMEM, st>>>(reinterpret_cast<float2 *>(spec), mf, gs,
+                                                                         reinterpret_cast<const float2 *>(ztw));
         }
     }
     template <int N> void zpass_launch(float gs) {
@@ -666,7 +703,7 @@ template <typename T, int R> struct PM : PMBase {
             }
             return CONAN_OK;
         } else {
-            return set_error(CONAN_ERR_UNSUPPORTED, "the z pass is FP32 only");
+            return line_green(gs);
         }
     }
 
@@ -822,15 +859,14 @@ template <typename T, int R> struct PM : PMBase {
     int poisson(double a) {
         const double gs = poisson_scale(a);
         if (zpass) {
-            // 2D R2C of every z plane, z pass with the Green multiply, 2D C2R
-            if constexpr (sizeof(T) == 4) {
-                CONAN_TIMED(prof, "fft_r2c", st, CONAN_TRY(fft2.forward(mesh, spec)));
-                CONAN_TRY(green_z(gs));
-                CONAN_TIMED(prof, "fft_c2r", st, CONAN_TRY(fft2.inverse(spec, mesh)));
-                CONAN_TRY(fd_gradient(mesh, grad));
-                mesh_holds = 2;
-                return CONAN_OK;
-            }
+            // the planes' (rows') R2C, the last axis with the Green multiply,
+            // the planes' C2R
+            CONAN_TIMED(prof, "fft_r2c", st, CONAN_TRY(fft2.forward(mesh, spec)));
+            CONAN_TRY(green_z(gs));
+            CONAN_TIMED(prof, "fft_c2r", st, CONAN_TRY(fft2.inverse(spec, mesh)));
+            CONAN_TRY(fd_gradient(mesh, grad));
+            mesh_holds = 2;
+            return CONAN_OK;
         }
         unsigned gb = (unsigned)((mf.spec + 255) / 256);
         CONAN_TIMED(prof, "fft_r2c", st, CONAN_TRY(fft.forward(mesh, spec)));
@@ -1025,7 +1061,7 @@ template <typename T, int R> struct PM : PMBase {
             tuned[tuned.size() - g.size() + best].chosen = true;
         }
         // (3) the z pass's lines per CTA (FP32 3D plane-transform solve)
-        if (zpass) {
+        if (zpass && sizeof(T) == 4) {
             const std::vector<int> w = zpass_widths();
             best = -1;
             bms = 1e30;
