@@ -419,6 +419,28 @@ __global__ void k_za_adjoint(T *db, const T *pb, size_t n, double cdz, double cp
     if (i < n) db[i] = (T)(cdz * (double)db[i] + cpz * (double)pb[i]);
 }
 
+// R arrays of n values copied at once, 16 bytes per thread and array
+// (cudaMalloc'd arrays). One launch instead of R copies, and faster than a
+// graph's copy nodes (a 512^3 model with two checkpoints: 39.5 ms against 40.9).
+template <typename T> struct CopyArrays {
+    const T *src[3];
+    T *dst[3];
+};
+template <typename T, int R> __global__ void __launch_bounds__(256) k_copy_arrays(CopyArrays<T> a, size_t n) {
+    constexpr int V = 16 / sizeof(T);
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (i + V <= n) {
+        uint4 v[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) v[k] = __ldcs(reinterpret_cast<const uint4 *>(a.src[k] + i));
+#pragma unroll
+        for (int k = 0; k < R; ++k) __stcs(reinterpret_cast<uint4 *>(a.dst[k] + i), v[k]);
+    } else {
+        for (int k = 0; k < R; ++k)
+            for (size_t j = i; j < n; ++j) a.dst[k][j] = a.src[k][j];
+    }
+}
+
 struct DiffBase {
     virtual ~DiffBase() {}
     virtual int forward(const void *noise, void *density, void *stream) = 0;
@@ -451,9 +473,17 @@ template <typename T, int R> struct Diff : DiffBase {
     // the gradient mesh is that of the final positions (forward's last step), as
     // backward's first step needs it
     bool grad_final = false;
+    // The launches of a pass between the caller's buffers, captured as graphs
+    // from a handle's second pass on (a few microseconds of host time per
+    // launch, and there are hundreds; building a graph pays from the second
+    // use). Everything in them belongs to the handle.
+    enum { G_STEPS, G_LAST, G_BACK, G_COUNT };
+    cudaGraphExec_t graphs[G_COUNT] = {};
+    unsigned graph_config = 0, passes[G_COUNT] = {};
 
     ~Diff() override {
         if (pm.st) cudaStreamSynchronize(pm.st);
+        drop_graphs();
         icfft.destroy();
         if (ev) cudaEventDestroy(ev);
     }
@@ -505,6 +535,45 @@ template <typename T, int R> struct Diff : DiffBase {
     unsigned kev() const { return prm.checkpoint_every ? prm.checkpoint_every : 1; }
     dim3 gp() const { return dim3((unsigned)((pm.np + 255) / 256)); }
 
+    void drop_graphs() {
+        for (auto &g : graphs) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+    }
+
+    // Enqueues what `body` launches on the handle's stream: directly the first
+    // time, as graph `which` from then on. body must leave the solver's host
+    // state as it finds it, apart from what the caller sets itself.
+    template <typename F> int replay(int which, F body) {
+        if (graph_config != pm.config) {  // other kernels were chosen meanwhile
+            drop_graphs();
+            graph_config = pm.config;
+        }
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;  // a caller's capture takes the launches themselves
+        CONAN_CUDA(cudaStreamIsCapturing(pm.st, &cs));
+        if (debug_sync() || cs != cudaStreamCaptureStatusNone || passes[which]++ == 0) return body();
+        if (!graphs[which]) {
+            cudaGraph_t g = nullptr;
+            CONAN_CUDA(cudaStreamBeginCapture(pm.st, cudaStreamCaptureModeThreadLocal));
+            const int rc = body();
+            const cudaError_t ce = cudaStreamEndCapture(pm.st, &g);
+            if (rc != CONAN_OK) {
+                if (g) cudaGraphDestroy(g);
+                return rc;
+            }
+            if (ce != cudaSuccess) return set_error(CONAN_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
+            const cudaError_t ie = cudaGraphInstantiate(&graphs[which], g, 0);
+            cudaGraphDestroy(g);
+            if (ie != cudaSuccess) {
+                graphs[which] = nullptr;
+                return set_error(CONAN_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ie));
+            }
+        }
+        CONAN_CUDA(cudaGraphLaunch(graphs[which], pm.st));
+        return CONAN_OK;
+    }
+
     // Orders the handle's stream after the caller's work. NULL is the legacy
     // default stream (where torch enqueues unless told otherwise), which a
     // non-blocking stream does not wait for by itself.
@@ -522,32 +591,43 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_CUDA(cudaStreamSynchronize(pm.st));
         return pm.check_err();
     }
+    int copy_arrays(T *const *dst, T *const *src) {
+        CopyArrays<T> c{};
+        for (int k = 0; k < R; ++k) {
+            c.src[k] = src[k];
+            c.dst[k] = dst[k];
+        }
+        const size_t nt = (pm.np * sizeof(T) + 15) / 16;
+        k_copy_arrays<T, R><<<(unsigned)((nt + 255) / 256), 256, 0, pm.st>>>(c, pm.np);
+        CONAN_LAUNCHED();
+        return CONAN_OK;
+    }
     // Positions (mom = false) or momenta of the current state into a slot.
     int save_ckpt(unsigned slot, bool mom) {
-        for (int k = 0; k < R; ++k)
-            CONAN_CUDA(cudaMemcpyAsync(ckpt[slot * 2 * R + (mom ? R : 0) + k], mom ? pm.P.p[k] : pm.P.d[k],
-                                       pm.np * sizeof(T), cudaMemcpyDeviceToDevice, pm.st));
-        return CONAN_OK;
+        return copy_arrays(&ckpt[slot * 2 * R + (mom ? R : 0)], mom ? pm.P.p : pm.P.d);
     }
     int load_ckpt(unsigned slot) {
         CONAN_TRY(pm.positions_reset());
-        for (int k = 0; k < R; ++k) {
-            CONAN_CUDA(cudaMemcpyAsync(pm.P.d[k], ckpt[slot * 2 * R + k], pm.np * sizeof(T), cudaMemcpyDeviceToDevice,
-                                       pm.st));
-            CONAN_CUDA(cudaMemcpyAsync(pm.P.p[k], ckpt[slot * 2 * R + R + k], pm.np * sizeof(T),
-                                       cudaMemcpyDeviceToDevice, pm.st));
-        }
-        return CONAN_OK;
+        CONAN_TRY(copy_arrays(pm.P.d, &ckpt[slot * 2 * R]));
+        return copy_arrays(pm.P.p, &ckpt[slot * 2 * R + R]);
     }
     double cdz() const { return -prm.a0 / (pm.res_m * pm.res_f); }
     double cpz() const { return -(prm.a0 + prm.da / 2) / (pm.res_m * pm.res_f); }
 
-    // Initial conditions of every member from the noise (device, batch) and
-    // the Zel'dovich start of the particle state at (a0, a0 + da/2).
-    int initial_state(const void *noise) {
-        cudaStream_t st = pm.st;
+    // The noise (device, batch) into the handle; what the solver had pending of
+    // other positions is dropped.
+    int take_noise(const void *noise) {
         grad_final = false;
-        CONAN_CUDA(cudaMemcpyAsync(w, noise, mm.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
+        CONAN_CUDA(cudaMemcpyAsync(w, noise, mm.cells * sizeof(T), cudaMemcpyDeviceToDevice, pm.st));
+        CONAN_TRY(pm.positions_reset());
+        pm.a_pos = prm.a0;
+        pm.a_mom = prm.a0 + prm.da / 2;
+        return CONAN_OK;
+    }
+    // Initial conditions of every member from the handle's noise and the
+    // Zel'dovich start of the particle state at (a0, a0 + da/2).
+    int start_state() {
+        cudaStream_t st = pm.st;
         for (int b = 0; b < mm.batch; ++b) {  // initial conditions, member by member
             T *x = ict + member_cells(mm, b);
             CONAN_TRY(grf_device<T>(ic[b], mm1, w + member_cells(mm, b), x, ics, icfft, part, st));
@@ -555,33 +635,47 @@ template <typename T, int R> struct Diff : DiffBase {
         }
         k_zeldovich<T, R><<<gp(), 256, 0, st>>>(pm.P, ict, mm, cdz(), cpz());
         CONAN_LAUNCHED();
-        CONAN_TRY(pm.positions_reset());
-        pm.a_pos = prm.a0;
-        pm.a_mom = prm.a0 + prm.da / 2;
         return CONAN_OK;
+    }
+    int initial_state(const void *noise) {
+        CONAN_TRY(take_noise(noise));
+        return start_state();
+    }
+
+    // The start and every step up to the last deposit. The kick of a step and
+    // the drift (with its deposit) of the next are one launch, as in a run; a
+    // checkpoint between them takes the positions before it (a kick moves
+    // none) and the momenta after it (a drift changes none).
+    int forward_steps() {
+        CONAN_TRY(start_state());
+        CONAN_TRY(save_ckpt(0, false));
+        CONAN_TRY(save_ckpt(0, true));
+        CONAN_TRY(pm.gkd(false, 0, true, pm.coef_drift(a_start[0], prm.da), true));
+        for (unsigned i = 0; i + 1 < prm.n; ++i) {
+            const double am = a_start[i] + prm.da / 2;
+            const bool save = (i + 1) % kev() == 0;
+            CONAN_TRY(pm.deposit_poisson(am));
+            if (save) CONAN_TRY(save_ckpt((i + 1) / kev(), false));
+            CONAN_TRY(pm.gkd(true, pm.coef_kick(am, prm.da), true, pm.coef_drift(a_start[i + 1], prm.da), true));
+            if (save) CONAN_TRY(save_ckpt((i + 1) / kev(), true));
+        }
+        return pm.deposit_for_solve();
+    }
+    int forward_last() {
+        const double am = a_start[prm.n - 1] + prm.da / 2;
+        CONAN_TRY(pm.solve_deposited(am));
+        return pm.gkd(true, pm.coef_kick(am, prm.da), false, 0, false);
     }
 
     int forward(const void *noise, void *density, void *stream) override {
         CONAN_TRY(enter(stream));
-        CONAN_TRY(initial_state(noise));
-        // The kick of a step and the drift (with its deposit) of the next are
-        // one launch, as in a run; a checkpoint between them takes the
-        // positions before it (a kick moves none) and the momenta after it
-        // (a drift changes none).
-        CONAN_TRY(save_ckpt(0, false));
-        CONAN_TRY(save_ckpt(0, true));
-        CONAN_TRY(pm.gkd(false, 0, true, pm.coef_drift(a_start[0], prm.da), true));
-        for (unsigned i = 0; i < prm.n; ++i) {
-            const double am = a_start[i] + prm.da / 2;
-            const bool last = i + 1 == prm.n, save = !last && (i + 1) % kev() == 0;
-            // the positions of the last deposit are the final ones: its
-            // density is the output
-            CONAN_TRY(pm.deposit_poisson(am, last ? (T *)density : nullptr));
-            if (save) CONAN_TRY(save_ckpt((i + 1) / kev(), false));
-            CONAN_TRY(pm.gkd(true, pm.coef_kick(am, prm.da), !last, last ? 0 : pm.coef_drift(a_start[i + 1], prm.da),
-                             !last));
-            if (save) CONAN_TRY(save_ckpt((i + 1) / kev(), true));
-        }
+        CONAN_TRY(take_noise(noise));
+        CONAN_TRY(replay(G_STEPS, [&] { return forward_steps(); }));
+        // the positions of the last deposit are the final ones: its density
+        // is the output
+        CONAN_TRY(pm.deposited_density((T *)density));
+        CONAN_TRY(replay(G_LAST, [&] { return forward_last(); }));
+        pm.mesh_holds = 2;
         grad_final = true;
         have_forward = true;
         return leave(stream);
@@ -635,15 +729,11 @@ template <typename T, int R> struct Diff : DiffBase {
         return CONAN_OK;
     }
 
-    int backward(const void *gdens, void *gnoise, void *stream) override {
-        if (!have_forward) return set_error(CONAN_ERR_STATE, "backward without a forward call");
-        CONAN_TRY(enter(stream));
+    // Every adjoint step from the density's adjoint in db. have_grad: the
+    // gradient mesh at the final positions is there from forward.
+    int backward_steps(bool have_grad) {
         cudaStream_t st = pm.st;
         const Mesh &mf = pm.mf;
-        const unsigned gc = (unsigned)((mf.cells + 255) / 256);
-        // the density adjoint through the final deposit
-        k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, (const T *)gdens, pm.mass, db[0], db[1], db[2]);
-        CONAN_LAUNCHED();
         for (int k = 0; k < R; ++k) CONAN_CUDA(cudaMemsetAsync(pb[k], 0, pm.np * sizeof(T), st));
         // the previous backward's first step left its maximum behind
         CONAN_CUDA(cudaMemsetAsync(absmax, 0, 4 * ABS_SLOTS * sizeof(unsigned long long), st));
@@ -652,8 +742,7 @@ template <typename T, int R> struct Diff : DiffBase {
             double ck = pm.coef_kick(am, prm.da), cd = pm.coef_drift(a, prm.da);
             // forward force at d_{i+1}: deposit, potential, gradient mesh
             // (the forward pass leaves the last step's)
-            if (!grad_final) CONAN_TRY(pm.deposit_poisson(am));
-            grad_final = false;
+            if (!have_grad || i != (int)prm.n - 1) CONAN_TRY(pm.deposit_poisson(am));
             // U = gather-transpose deposit of v = pbar and the density's
             // adjoint rhobar; pbar is zero in the last step (the loss sees
             // positions only), and so is rhobar
@@ -671,6 +760,22 @@ template <typename T, int R> struct Diff : DiffBase {
             CONAN_LAUNCHED();
             if ((unsigned)i % kev() == 0) CONAN_TRY(load_ckpt((unsigned)i / kev()));
         }
+        return CONAN_OK;
+    }
+
+    int backward(const void *gdens, void *gnoise, void *stream) override {
+        if (!have_forward) return set_error(CONAN_ERR_STATE, "backward without a forward call");
+        CONAN_TRY(enter(stream));
+        cudaStream_t st = pm.st;
+        const Mesh &mf = pm.mf;
+        const unsigned gc = (unsigned)((mf.cells + 255) / 256);
+        // the density adjoint through the final deposit
+        k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, (const T *)gdens, pm.mass, db[0], db[1], db[2]);
+        CONAN_LAUNCHED();
+        if (grad_final) CONAN_TRY(replay(G_BACK, [&] { return backward_steps(true); }));
+        else CONAN_TRY(backward_steps(false));
+        grad_final = false;
+        pm.mesh_holds = 2;
         // Zel'dovich, potential and random-field adjoints on the mass mesh
         unsigned gm = (unsigned)((mm.cells + 255) / 256);
         for (int k = 0; k < R; ++k) {

@@ -272,6 +272,7 @@ template <typename T, int R> struct PM : PMBase {
     // DEP_LAG: Lagrangian-window deposit (FP32). Chosen by the autotuner.
     static constexpr int DEP_LAG = DEP_VARIANTS;
     int dep_variant = 0;
+    unsigned config = 0;  // changes of the kernels' choice: what was captured before is stale
 
     // Lagrangian deposit: accumulator mesh, lattice-tile variant and window.
     unsigned long long *lacc = nullptr;
@@ -514,6 +515,7 @@ template <typename T, int R> struct PM : PMBase {
     // CONAN_DEPOSIT_SORTED or CONAN_DEPOSIT_LAGRANGIAN.
     int set_deposit(int mode) override {
         CONAN_TRY(drop_lag_deposit());  // a pending fused deposit belongs to the old mode
+        ++config;
         if (mode == CONAN_DEPOSIT_SORTED) {
             dep_variant = dep_default();
             return CONAN_OK;
@@ -830,24 +832,28 @@ template <typename T, int R> struct PM : PMBase {
     }
 
     // The deposit of the current positions and the Poisson solve of the
-    // kick that follows it: through the cluster plane pass when it is on,
-    // else deposit() (density mesh) and poisson().
-    // delta_out (device, may be null) receives the density contrast.
-    int deposit_poisson(double a, T *delta_out = nullptr) {
-        if (plane_on()) {
-            CONAN_TRY(lag_accumulate());
-            if (delta_out) CONAN_TRY(acc_mesh(delta_out));
-            const double gs = poisson_scale(a);
-            if (mf.n == 512) CONAN_TRY((plane_kc == 16 ? plane_run<512, 16>(gs) : plane_run<512, 32>(gs)));
-            else CONAN_TRY((plane_kc == 16 ? plane_run<256, 16>(gs) : plane_run<256, 32>(gs)));
-            CONAN_TRY(fd_gradient(mesh, grad));
-            mesh_holds = 2;
-            return CONAN_OK;
-        }
-        CONAN_TRY(deposit());
-        if (delta_out)
-            CONAN_CUDA(cudaMemcpyAsync(delta_out, mesh, mf.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        return poisson(a);
+    // kick that follows it: through the cluster plane pass when it is on
+    // (which reads the accumulator itself), else deposit() (density mesh) and
+    // poisson().
+    int deposit_for_solve() { return plane_on() ? lag_accumulate() : deposit(); }
+    int solve_deposited(double a) {
+        if (!plane_on()) return poisson(a);
+        const double gs = poisson_scale(a);
+        if (mf.n == 512) CONAN_TRY((plane_kc == 16 ? plane_run<512, 16>(gs) : plane_run<512, 32>(gs)));
+        else CONAN_TRY((plane_kc == 16 ? plane_run<256, 16>(gs) : plane_run<256, 32>(gs)));
+        CONAN_TRY(fd_gradient(mesh, grad));
+        mesh_holds = 2;
+        return CONAN_OK;
+    }
+    // Between the two: the density contrast into out (device).
+    int deposited_density(T *out) {
+        if (plane_on()) return acc_mesh(out);
+        CONAN_CUDA(cudaMemcpyAsync(out, mesh, mf.cells * sizeof(T), cudaMemcpyDeviceToDevice, st));
+        return CONAN_OK;
+    }
+    int deposit_poisson(double a) {
+        CONAN_TRY(deposit_for_solve());
+        return solve_deposited(a);
     }
 
     // Green's function factor of a kick at a, with the per-member
@@ -988,6 +994,7 @@ template <typename T, int R> struct PM : PMBase {
         const bool prof_was = prof.on;
         prof.on = false;
         int rc = tune_knobs(save.data(), a, da);
+        ++config;
         prof.on = prof_was;
         for (int k = 0; k < R && rc == CONAN_OK; ++k) {
             cudaMemcpyAsync(P.d[k], save[k], np * sizeof(T), cudaMemcpyDeviceToDevice, st);
