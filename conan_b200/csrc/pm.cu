@@ -211,6 +211,11 @@ template <typename T, int R> struct PM : PMBase {
             pers = LAG_PERSIST != 0;
             CONAN_TRY(pers_setup());
         }
+        if (sizeof(T) == 8 && np <= DIRECT_MAX && mf.cells <= DIRECT_MAX) {
+            CONAN_TRY(alloc(&dacc, mf.cells));
+            CONAN_CUDA(cudaMemsetAsync(dacc, 0, mf.cells * sizeof(ulonglong2), st));
+            dep_variant = DEP_DIRECT;
+        }
         CONAN_TRY(fft.create(mf, sizeof(T) == 8, batch));
         size_t wbytes = fft.work_bytes;
         const bool split = sizeof(T) == 4 ? R == 3 && mf.n <= 1024 : (R == 3 && mf.n <= 512) || (R == 2 && mf.n <= 1024);
@@ -265,12 +270,22 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
+    // Largest lattice and mesh whose FP64 deposit goes straight to the
+    // accumulator by default: up to there the counting sort's five launches
+    // cost more than the atomics (per FP64 step, 2D 256^2 31 -> 21 us, 1024^2
+    // 108 -> 104, 3D 64^3 64 -> 52; 128^3 286 against 280 us, 307 against 316
+    // where clustered, and 256^3 1.94 against 2.19 ms).
+    static constexpr size_t DIRECT_MAX = (size_t)1 << 20;
+
     dim3 grid_p() const { return dim3((unsigned)((np + 255) / 256)); }
 
     // --- deposit ---------------------------------------------------------
     // 0 .. DEP_VARIANTS-1: sorted deposit with tile shape DepTile<R, V>;
     // DEP_LAG: Lagrangian-window deposit (FP32). Chosen by the autotuner.
-    static constexpr int DEP_LAG = DEP_VARIANTS;
+    // DEP_DIRECT: corners straight into a two-word accumulator (FP64, small
+    // lattices; reported as the sorted deposit, whose bits it has, and left for
+    // good when the caller asks for that one by name).
+    static constexpr int DEP_LAG = DEP_VARIANTS, DEP_DIRECT = DEP_LAG + 1;
     int dep_variant = 0;
     unsigned config = 0;  // changes of the kernels' choice: what was captured before is stale
 
@@ -279,6 +294,9 @@ template <typename T, int R> struct PM : PMBase {
     int lag_v = -1;  // LagTile<R, V> variant that fits this mesh, -1: none
     LagWin lwin{};
     size_t lag_smem = 0;
+
+    ulonglong2 *dacc = nullptr;  // direct FP64 deposit
+    bool direct_on() const { return sizeof(T) == 8 && dep_variant == DEP_DIRECT && dacc; }
 
     bool lag_on() const { return sizeof(T) == 4 && dep_variant == DEP_LAG && lag_v >= 0 && lacc; }
 
@@ -464,7 +482,10 @@ template <typename T, int R> struct PM : PMBase {
     // made by the fused kernel and not yet turned into the density mesh.
     bool lag_ready = false;
     int drop_lag_deposit() {
-        if (lag_ready) CONAN_CUDA(cudaMemsetAsync(lacc, 0, mf.cells * sizeof(unsigned long long), st));
+        if (lag_ready) {
+            if (direct_on()) CONAN_CUDA(cudaMemsetAsync(dacc, 0, mf.cells * sizeof(ulonglong2), st));
+            else CONAN_CUDA(cudaMemsetAsync(lacc, 0, mf.cells * sizeof(unsigned long long), st));
+        }
         lag_ready = false;
         return CONAN_OK;
     }
@@ -568,6 +589,18 @@ template <typename T, int R> struct PM : PMBase {
 
     int deposit() {
         if (lag_on()) return deposit_lag();
+        if constexpr (sizeof(T) == 8) {
+            if (direct_on()) {
+                if (!lag_ready)
+                    CONAN_TIMED(prof, "deposit", st, (k_deposit_direct<R><<<grid_p(), 256, 0, st>>>(P, mf, dacc)));
+                lag_ready = false;
+                CONAN_TIMED(prof, "deposit_mesh", st,
+                            (k_direct_mesh<<<(unsigned)((mf.cells + 255) / 256), 256, 0, st>>>(dacc, mesh, mf.cells,
+                                                                                                mass)));
+                mesh_holds = 1;
+                return CONAN_OK;
+            }
+        }
         if (!ranks_pending) CONAN_TRY(rank_pass());
         CONAN_TIMED(prof, "scan", st, scan_exclusive(count, mf.cells, bsum, off, st));
         ranks_pending = false;
@@ -930,7 +963,7 @@ template <typename T, int R> struct PM : PMBase {
     std::vector<TuneRec> tuned;
     static constexpr int TUNE_STEPS = 2;
     struct DepCand {
-        int mode;  // 0 sorted, 1 Lagrangian window, 2 Lagrangian direct, 3 Lagrangian window, persistent
+        int mode;  // 0 sorted (v = DEP_DIRECT: direct FP64), 1 Lagrangian window, 2 Lagrangian direct, 3 Lagrangian window, persistent
         int v;
         std::string name;
     };
@@ -1017,6 +1050,7 @@ template <typename T, int R> struct PM : PMBase {
         if (dep_fits<1>()) cands.push_back({0, 1, "sorted 32x4x8 / 128 threads"});
         if (dep_fits<2>()) cands.push_back({0, 2, "sorted 32x16x8 / 512 threads"});
         if (dep_fits<DEP_SMALL>()) cands.push_back({0, DEP_SMALL, "sorted, tiles of 256 cells / 256 threads"});
+        if (dacc) cands.push_back({0, DEP_DIRECT, "direct, two words per cell"});
         if (sizeof(T) == 4 && lacc) {
             const char *tile[4] = {"", "", "", ""};
             if (R == 3) tile[0] = "32x8x8", tile[1] = "16x8x8", tile[2] = "8x8x8", tile[3] = "16x8x4";
@@ -1144,7 +1178,8 @@ template <typename T, int R> struct PM : PMBase {
     // drift, the deposit itself in the same kernel).
     int gkd(bool kick, double ck, bool drift, double cd, bool rank_after) {
         const bool fuse = rank_after && drift && lag_on() && prm.gradient == CONAN_GRAD_FD4;
-        rank_after = rank_after && !lag_on();  // the Lagrangian deposit needs no ranks
+        const bool direct = rank_after && drift && direct_on();
+        rank_after = rank_after && !lag_on() && !direct_on();  // these deposits need no ranks
         // ranks of positions about to move are stale either way
         if ((rank_after || drift) && ranks_pending) {
             CONAN_CUDA(cudaMemsetAsync(count, 0, mf.cells * sizeof(uint32_t), st));
@@ -1172,15 +1207,17 @@ template <typename T, int R> struct PM : PMBase {
             else CONAN_TRY(launch_gkd_lag<3>(c, name));
             return CONAN_OK;
         }
+        ulonglong2 *const da = direct ? dacc : nullptr;
         if (prm.gradient == CONAN_GRAD_SPECTRAL)
             CONAN_TIMED(prof, name, st,
                         (k_gkd<T, R, true><<<grid_p(), 256, 0, st>>>(P, mf, mesh, gm[0], gm[1], gm[2], grad, c,
-                                                                     count, rank)));
+                                                                     count, rank, da)));
         else
             CONAN_TIMED(prof, name, st,
                         (k_gkd<T, R, false><<<grid_p(), 256, 0, st>>>(P, mf, mesh, gm[0], gm[1], gm[2], grad, c,
-                                                                      count, rank)));
+                                                                      count, rank, da)));
         if (rank_after) ranks_pending = true;
+        if (direct) lag_ready = true;
         return CONAN_OK;
     }
 

@@ -733,14 +733,71 @@ struct GKD {
     int deposit = 1;  // fused Lagrangian tiles: deposit the drifted positions (0: kick and/or drift only)
 };
 
+// ------------------------------------------------ FP64 direct deposit --
+//
+// On small lattices the FP64 deposit's counting sort is five launches of a few
+// microseconds each. Here every corner goes straight into an accumulator of
+// two 64-bit words per cell: the low 32 bits of its weight in units of 2^-52
+// into one, the rest into the other, which hold any number of particles below
+// 2^31 without a carry. The sums are the sorted deposit's 96-bit ones, so the
+// density has the same bits.
+template <int R>
+__device__ inline void direct_add(const Parts<double> &P, const Mesh &m, size_t i, const double *d,
+                                  ulonglong2 *__restrict__ acc) {
+    int q[3], cell[3];
+    double fr[3];
+    lattice<double, R>(P, i, q);
+#pragma unroll
+    for (int k = 0; k < R; ++k) Pay<double>::cell_frac(d[k], q[k], m.n - 1, &cell[k], &fr[k]);
+    acc += cell_base(P, m, i);
+    const double wx[2] = {1.0 - fr[0], fr[0]};
+    const double wy[2] = {R >= 2 ? 1.0 - fr[1] : 1.0, R >= 2 ? fr[1] : 1.0};
+    const double wz[2] = {R == 3 ? 1.0 - fr[2] : 1.0, R == 3 ? fr[2] : 1.0};
+#pragma unroll
+    for (int b = 0; b < (1 << R); ++b) {
+        uint32_t ci = 0;
+#pragma unroll
+        for (int k = R - 1; k >= 0; --k) ci = (ci << m.shift) | (uint32_t)((cell[k] + ((b >> k) & 1)) & (m.n - 1));
+        const unsigned long long v = quant_w(wx[b & 1] * wy[(b >> 1) & 1] * wz[(b >> 2) & 1]);
+        unsigned long long *p = reinterpret_cast<unsigned long long *>(acc + ci);
+        if (v & 0xffffffffull) atomicAdd(p, v & 0xffffffffull);
+        if (v >> 32) atomicAdd(p + 1, v >> 32);
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_deposit_direct(Parts<double> P, Mesh m, ulonglong2 *__restrict__ acc) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.np) return;
+    double d[3];
+#pragma unroll
+    for (int k = 0; k < R; ++k) d[k] = P.d[k][i];
+    direct_add<R>(P, m, i, d, acc);
+}
+
+// Density contrast from the two-word accumulator, as the sorted deposit forms
+// it from its three words; the accumulator is left clear.
+static __global__ void __launch_bounds__(256) k_direct_mesh(ulonglong2 *__restrict__ acc, double *__restrict__ out, size_t n,
+                                                     double scale) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const ulonglong2 a = acc[i];
+    acc[i] = make_ulonglong2(0ull, 0ull);
+    const unsigned long long hi = a.y + (a.x >> 32);
+    const double v = (double)(uint32_t)(hi >> 32) * 0x1p12 + (double)(uint32_t)hi * 0x1p-20 +
+                     (double)(uint32_t)a.x * 0x1p-52;
+    out[i] = v * scale - 1.0;
+}
+
 // Fused leapfrog update of particle i: the kick of Gravity::kick
 // (src/run/nbody.hh:112-117), then the next step's drift (Gravity::drift,
 // src/run/nbody.hh:122-130), then the counting-sort rank of the new cell.
+// or (FP64 with a direct accumulator dacc) the deposit of the new position.
 template <typename T, int R, bool SPECTRAL>
 __global__ void __launch_bounds__(256)
     k_gkd(Parts<T> P, Mesh m, const T *__restrict__ phi, const T *__restrict__ g0,
           const T *__restrict__ g1, const T *__restrict__ g2, const G4<T> *__restrict__ G, GKD c,
-          uint32_t *__restrict__ count, uint32_t *__restrict__ rank) {
+          uint32_t *__restrict__ count, uint32_t *__restrict__ rank, ulonglong2 *__restrict__ dacc) {
     size_t i = tiled_index<T, R>(P, blockIdx.x, threadIdx.x);
     if (i >= P.np) return;
     T d[3], p[3];
@@ -767,6 +824,9 @@ __global__ void __launch_bounds__(256)
             d[k] += p[k] * cd;
             P.d[k][i] = d[k];
         }
+    }
+    if constexpr (sizeof(T) == 8) {
+        if (dacc) direct_add<R>(P, m, i, d, dacc);
     }
     if (c.rank) rank[i] = atomicAdd(count + cell_base(P, m, i) + deposit_cell<T, R>(P, m, i), 1u);
 }
