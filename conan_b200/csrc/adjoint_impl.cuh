@@ -412,11 +412,24 @@ __global__ void __launch_bounds__(256, 4)
     absmax_add(absmax, lanes, (blockIdx.x * 8 + (threadIdx.x >> 5)) % ABS_SLOTS, mx);
 }
 
-// ubar_k = cdz dbar_k + cpz pbar_k in place in dbar (particle i = mass cell i).
-template <typename T>
-__global__ void k_za_adjoint(T *db, const T *pb, size_t n, double cdz, double cpz) {
+// ubar_k = cdz dbar_k + cpz pbar_k in place in dbar (particle i = mass cell
+// i), all axes in one launch.
+template <typename T, int R> struct ZaArrays {
+    T *db[3];
+    const T *pb[3];
+};
+template <typename T, int R>
+__global__ void __launch_bounds__(256) k_za_adjoint(ZaArrays<T, R> a, size_t n, double cdz, double cpz) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) db[i] = (T)(cdz * (double)db[i] + cpz * (double)pb[i]);
+    if (i >= n) return;
+    T d[R], p[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        d[k] = a.db[k][i];
+        p[k] = a.pb[k][i];
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) a.db[k][i] = (T)(cdz * (double)d[k] + cpz * (double)p[k]);
 }
 
 // R arrays of n values copied at once, 16 bytes per thread and array
@@ -507,10 +520,13 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_TRY(icfft.create(mm1, sizeof(T) == 8, 1));
         CONAN_TRY(pm.alloc((char **)&icwork, icfft.work_bytes ? icfft.work_bytes : 16));
         CONAN_TRY(icfft.bind(icwork, pm.st));
+        // pb and U in one piece each: one memset clears all their axes
+        CONAN_TRY(pm.alloc(&pb[0], R * pm.np));
+        CONAN_TRY(pm.alloc(&U[0], R * pm.mf.cells));
         for (int k = 0; k < R; ++k) {
             CONAN_TRY(pm.alloc(&db[k], pm.np));
-            CONAN_TRY(pm.alloc(&pb[k], pm.np));
-            CONAN_TRY(pm.alloc(&U[k], pm.mf.cells));
+            pb[k] = pb[0] + k * pm.np;
+            U[k] = U[0] + k * pm.mf.cells;
         }
         CONAN_TRY(pm.alloc(&rhobar, pm.mf.cells));
         CONAN_TRY(pm.alloc(&S, 1));
@@ -684,7 +700,7 @@ template <typename T, int R> struct Diff : DiffBase {
     template <typename UT> int neg_div(UT *const *u, const int *exps, T *out, const Mesh &m) {
         if constexpr (R == 3) {
             if (m.n >= 32) {
-                const unsigned blocks = (unsigned)((size_t)(m.n / 32) * (m.n / 8) * (m.n / NDZ) * m.batch);
+                const unsigned blocks = (unsigned)(m.cells / (256 * NDZ));
                 k_neg_div_z<T, UT><<<blocks, 256, 0, pm.st>>>(u[0], u[1], u[2], exps, out, m);
                 CONAN_LAUNCHED();
                 return CONAN_OK;
@@ -734,7 +750,7 @@ template <typename T, int R> struct Diff : DiffBase {
     int backward_steps(bool have_grad) {
         cudaStream_t st = pm.st;
         const Mesh &mf = pm.mf;
-        for (int k = 0; k < R; ++k) CONAN_CUDA(cudaMemsetAsync(pb[k], 0, pm.np * sizeof(T), st));
+        CONAN_CUDA(cudaMemsetAsync(pb[0], 0, R * pm.np * sizeof(T), st));
         // the previous backward's first step left its maximum behind
         CONAN_CUDA(cudaMemsetAsync(absmax, 0, 4 * ABS_SLOTS * sizeof(unsigned long long), st));
         for (int i = (int)prm.n - 1; i >= 0; --i) {
@@ -750,8 +766,7 @@ template <typename T, int R> struct Diff : DiffBase {
             if (!vz) {
                 k_fix_exponent<<<1, ABS_SLOTS, 0, st>>>(absmax, (double)pm.np, R, S);
                 CONAN_LAUNCHED();
-                for (int k = 0; k < R; ++k)
-                    CONAN_CUDA(cudaMemsetAsync(U[k], 0, mf.cells * sizeof(unsigned long long), st));
+                CONAN_CUDA(cudaMemsetAsync(U[0], 0, R * mf.cells * sizeof(unsigned long long), st));
                 CONAN_TRY(vec_deposit());
                 CONAN_TRY(adjoint_poisson(am));
             }
@@ -778,10 +793,13 @@ template <typename T, int R> struct Diff : DiffBase {
         pm.mesh_holds = 2;
         // Zel'dovich, potential and random-field adjoints on the mass mesh
         unsigned gm = (unsigned)((mm.cells + 255) / 256);
+        ZaArrays<T, R> za{};
         for (int k = 0; k < R; ++k) {
-            k_za_adjoint<T><<<gm, 256, 0, st>>>(db[k], pb[k], mm.cells, cdz(), cpz());
-            CONAN_LAUNCHED();
+            za.db[k] = db[k];
+            za.pb[k] = pb[k];
         }
+        k_za_adjoint<T, R><<<gm, 256, 0, st>>>(za, mm.cells, cdz(), cpz());
+        CONAN_LAUNCHED();
         CONAN_TRY(neg_div(db, nullptr, ict, mm));
         for (int b = 0; b < mm.batch; ++b) {
             const size_t o = member_cells(mm, b);

@@ -951,7 +951,7 @@ template <typename T, int R> struct PM : PMBase {
     // particles cluster) it chooses (1) the deposit: the sorted tile variants,
     // the Lagrangian window tiles V0..V2 and the direct two-cell window
     // (FP32); (2) the gradient-mesh kernel: one thread per cell in blocks of
-    // 128, 256 or 512, or z-marching tiles. Knobs are tuned one after the
+    // 128, 256 or 512, or z-marching columns. Knobs are tuned one after the
     // other; each candidate runs one untimed and TUNE_STEPS timed leapfrog
     // steps (CUDA events) from a copy of the state, which is restored at the
     // end.
