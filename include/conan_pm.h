@@ -279,7 +279,7 @@ int conan_pm_get_stream(conan_pm *h, void **stream);
  * the state and keeps the fastest: the deposit (sorted tile variants;
  * Lagrangian window tiles; the direct two-cell window) and the
  * gradient-mesh kernel (thread per cell at 128/256/512 threads; z-marching
- * tiles). a: scale factor of the next drift; da: the step. The state and
+ * columns). a: scale factor of the next drift; da: the step. The state and
  * scale factors are left as they were. `report` (may be NULL) receives a
  * JSON list of {knob, value, ms_per_step, chosen}. Allocates a temporary
  * copy of the particle state. */
