@@ -1458,7 +1458,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 // Density contrast from the integer accumulator (units of 2^-23 particle
 // weights): out = sum 2^-23 mass - 1, as the sorted deposit. The caller
 // clears the accumulator afterwards (a plain memset streams faster than
-// zero stores mixed into this read stream).
+// zero stores mixed into this read stream). out may be a caller's array, which
+// need only be aligned as a T: 16-byte stores where its address allows them.
 template <typename T>
 __global__ void __launch_bounds__(256) k_acc_mesh(unsigned long long *__restrict__ acc, T *__restrict__ out,
                                                   size_t n, double scale) {
@@ -1469,8 +1470,8 @@ __global__ void __launch_bounds__(256) k_acc_mesh(unsigned long long *__restrict
         const double k = 0x1p-23 * scale;
         T v0 = (T)((double)a.x * k - 1.0), v1 = (T)((double)a.y * k - 1.0);
         T v2 = (T)((double)b.x * k - 1.0), v3 = (T)((double)b.y * k - 1.0);
-        if constexpr (sizeof(T) == 4) {
-            *reinterpret_cast<float4 *>(out + i) = make_float4(v0, v1, v2, v3);
+        if (sizeof(T) == 4 && ((uintptr_t)out & 15) == 0) {
+            *reinterpret_cast<float4 *>(out + i) = make_float4((float)v0, (float)v1, (float)v2, (float)v3);
         } else {
             out[i] = v0;
             out[i + 1] = v1;
