@@ -10,7 +10,8 @@ potential, Zel'dovich start), n leapfrog steps and the final CIC deposit on
 the GPU; backward runs the adjoint of all of it (reversible leapfrog with an
 exact checkpoint every `checkpoint_every` steps). Tensors are flat with axis
 0 fastest, the reference's mesh layout. One model holds the state of its last
-forward: call backward before the next forward of the same model.
+forward: call backward (as often as there are losses) before the next forward of
+the same model.
 """
 from __future__ import annotations
 

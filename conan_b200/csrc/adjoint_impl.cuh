@@ -482,10 +482,11 @@ template <typename T, int R> struct Diff : DiffBase {
     std::vector<T *> ckpt;  // per checkpoint: d[0..R), p[0..R)
     std::vector<double> a_start;
     cudaEvent_t ev = nullptr;
-    bool have_forward = false;
-    // the gradient mesh is that of the final positions (forward's last step), as
-    // backward's first step needs it
-    bool grad_final = false;
+    bool have_forward = false;  // the checkpoints are those of a forward that was enqueued whole
+    // the state is the final one and the gradient mesh that of the last step,
+    // as forward leaves them and backward starts from (it ends at the initial
+    // state)
+    bool at_final = false;
     // The launches of a pass between the caller's buffers, captured as graphs
     // from a handle's second pass on (a few microseconds of host time per
     // launch, and there are hundreds; building a graph pays from the second
@@ -633,7 +634,7 @@ template <typename T, int R> struct Diff : DiffBase {
     // The noise (device, batch) into the handle; what the solver had pending of
     // other positions is dropped.
     int take_noise(const void *noise) {
-        grad_final = false;
+        have_forward = at_final = false;
         CONAN_CUDA(cudaMemcpyAsync(w, noise, mm.cells * sizeof(T), cudaMemcpyDeviceToDevice, pm.st));
         CONAN_TRY(pm.positions_reset());
         pm.a_pos = prm.a0;
@@ -658,16 +659,13 @@ template <typename T, int R> struct Diff : DiffBase {
         return start_state();
     }
 
-    // The start and every step up to the last deposit. The kick of a step and
-    // the drift (with its deposit) of the next are one launch, as in a run; a
-    // checkpoint between them takes the positions before it (a kick moves
+    // From the state before step i0 up to the last deposit. The kick of a step
+    // and the drift (with its deposit) of the next are one launch, as in a run;
+    // a checkpoint between them takes the positions before it (a kick moves
     // none) and the momenta after it (a drift changes none).
-    int forward_steps() {
-        CONAN_TRY(start_state());
-        CONAN_TRY(save_ckpt(0, false));
-        CONAN_TRY(save_ckpt(0, true));
-        CONAN_TRY(pm.gkd(false, 0, true, pm.coef_drift(a_start[0], prm.da), true));
-        for (unsigned i = 0; i + 1 < prm.n; ++i) {
+    int steps_from(unsigned i0) {
+        CONAN_TRY(pm.gkd(false, 0, true, pm.coef_drift(a_start[i0], prm.da), true));
+        for (unsigned i = i0; i + 1 < prm.n; ++i) {
             const double am = a_start[i] + prm.da / 2;
             const bool save = (i + 1) % kev() == 0;
             CONAN_TRY(pm.deposit_poisson(am));
@@ -677,10 +675,24 @@ template <typename T, int R> struct Diff : DiffBase {
         }
         return pm.deposit_for_solve();
     }
+    int forward_steps() {
+        CONAN_TRY(start_state());
+        CONAN_TRY(save_ckpt(0, false));
+        CONAN_TRY(save_ckpt(0, true));
+        return steps_from(0);
+    }
     int forward_last() {
         const double am = a_start[prm.n - 1] + prm.da / 2;
         CONAN_TRY(pm.solve_deposited(am));
         return pm.gkd(true, pm.coef_kick(am, prm.da), false, 0, false);
+    }
+    // The final state again, from the last checkpoint: the forward's own
+    // launches from there, so its bits.
+    int restore_final() {
+        const unsigned slot = (prm.n - 1) / kev();
+        CONAN_TRY(load_ckpt(slot));
+        CONAN_TRY(steps_from(slot * kev()));
+        return forward_last();
     }
 
     int forward(const void *noise, void *density, void *stream) override {
@@ -692,8 +704,7 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_TRY(pm.deposited_density((T *)density));
         CONAN_TRY(replay(G_LAST, [&] { return forward_last(); }));
         pm.mesh_holds = 2;
-        grad_final = true;
-        have_forward = true;
+        at_final = have_forward = true;
         return leave(stream);
     }
 
@@ -745,9 +756,9 @@ template <typename T, int R> struct Diff : DiffBase {
         return CONAN_OK;
     }
 
-    // Every adjoint step from the density's adjoint in db. have_grad: the
-    // gradient mesh at the final positions is there from forward.
-    int backward_steps(bool have_grad) {
+    // Every adjoint step from the density's adjoint in db, the final state
+    // and its gradient mesh back to the initial state.
+    int backward_steps() {
         cudaStream_t st = pm.st;
         const Mesh &mf = pm.mf;
         CONAN_CUDA(cudaMemsetAsync(pb[0], 0, R * pm.np * sizeof(T), st));
@@ -756,14 +767,13 @@ template <typename T, int R> struct Diff : DiffBase {
         for (int i = (int)prm.n - 1; i >= 0; --i) {
             double a = a_start[i], am = a + prm.da / 2;
             double ck = pm.coef_kick(am, prm.da), cd = pm.coef_drift(a, prm.da);
-            // forward force at d_{i+1}: deposit, potential, gradient mesh
-            // (the forward pass leaves the last step's)
-            if (!have_grad || i != (int)prm.n - 1) CONAN_TRY(pm.deposit_poisson(am));
-            // U = gather-transpose deposit of v = pbar and the density's
-            // adjoint rhobar; pbar is zero in the last step (the loss sees
-            // positions only), and so is rhobar
+            // forward force at d_{i+1}: deposit, potential, gradient mesh (the
+            // last step's is there). U = gather-transpose deposit of v = pbar
+            // and the density's adjoint rhobar; pbar is zero in the last step
+            // (the loss sees positions only), and so is rhobar
             const bool vz = i == (int)prm.n - 1;
             if (!vz) {
+                CONAN_TRY(pm.deposit_poisson(am));
                 k_fix_exponent<<<1, ABS_SLOTS, 0, st>>>(absmax, (double)pm.np, R, S);
                 CONAN_LAUNCHED();
                 CONAN_CUDA(cudaMemsetAsync(U[0], 0, R * mf.cells * sizeof(unsigned long long), st));
@@ -782,14 +792,12 @@ template <typename T, int R> struct Diff : DiffBase {
         if (!have_forward) return set_error(CONAN_ERR_STATE, "backward without a forward call");
         CONAN_TRY(enter(stream));
         cudaStream_t st = pm.st;
-        const Mesh &mf = pm.mf;
-        const unsigned gc = (unsigned)((mf.cells + 255) / 256);
+        if (!at_final) CONAN_TRY(restore_final());  // a further gradient of the same forward
+        at_final = false;
         // the density adjoint through the final deposit
-        k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, mf, (const T *)gdens, pm.mass, db[0], db[1], db[2]);
+        k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, pm.mf, (const T *)gdens, pm.mass, db[0], db[1], db[2]);
         CONAN_LAUNCHED();
-        if (grad_final) CONAN_TRY(replay(G_BACK, [&] { return backward_steps(true); }));
-        else CONAN_TRY(backward_steps(false));
-        grad_final = false;
+        CONAN_TRY(replay(G_BACK, [&] { return backward_steps(); }));
         pm.mesh_holds = 2;
         // Zel'dovich, potential and random-field adjoints on the mass mesh
         unsigned gm = (unsigned)((mm.cells + 255) / 256);
@@ -807,7 +815,6 @@ template <typename T, int R> struct Diff : DiffBase {
             CONAN_TRY(grf_adjoint_device<T>(ic[b], mm1, w + o, ict + o, (T *)gnoise + o, ics, ics2, ict2, icfft,
                                             part, st));
         }
-        (void)gc;
         return leave(stream);
     }
 };

@@ -307,7 +307,9 @@ void conan_diff_destroy(conan_diff *h);
  * later work on it after the call (with NULL the call waits for its work). */
 int conan_diff_forward(conan_diff *h, const void *noise_dev, void *density_out_dev, void *stream);
 /* Gradient of a scalar loss w.r.t. the noise given its gradient w.r.t. the
- * final density of the last forward call. */
+ * final density of the last forward call. Further calls give the gradients of
+ * other losses of the same forward (each first runs the steps from the last
+ * checkpoint again). */
 int conan_diff_backward(conan_diff *h, const void *grad_density_dev, void *grad_noise_dev,
                         void *stream);
 

@@ -24,3 +24,31 @@ def test_density_arrays_need_no_more_than_a_floats_alignment(gpu, conan, monkeyp
         assert torch.equal(buf[skip:skip + m.ncells], ref)
         assert (buf[:skip] == 7).all() and (buf[skip + m.ncells:] == 7).all()
     m.close()
+
+
+# the last checkpoint at the initial state, one step and several before the end
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("mbits,n,every", [(4, 3, 8), (5, 5, 2), (6, 4, 2), (6, 1, 1)])
+def test_a_further_gradient_of_one_forward(gpu, conan, prec, mbits, n, every):
+    from conan_b200.autograd import DiffPM
+    dt = torch.float32 if prec == "fp32" else torch.float64
+    m = DiffPM(dim=3, mbits=mbits, L_box=60.0, ns=-2.0, a0=0.05, da=0.08, n=n, checkpoint_every=every, precision=prec)
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    noise = torch.randn(m.nnoise, device="cuda", dtype=dt, generator=gen)
+    losses = [torch.randn(m.ncells, device="cuda", dtype=dt, generator=gen) / m.ncells for _ in range(3)]
+    out, g = torch.empty_like(losses[0]), torch.empty_like(noise)
+    want = []
+    for gd in losses:  # one forward each
+        m.forward_raw(noise, out)
+        m.backward_raw(gd, g)
+        want.append(g.clone())
+    m.forward_raw(noise, out)
+    for gd, w in list(zip(losses, want)) + [(losses[0], want[0])]:  # one forward for all
+        m.backward_raw(gd, g)
+        assert torch.equal(g, w)
+    # through torch.autograd: two losses of one density
+    x = noise.clone().requires_grad_(True)
+    delta = m(x)
+    for gd, w in zip(losses[:2], want):
+        assert torch.equal(torch.autograd.grad(delta, x, gd, retain_graph=True)[0], w)
+    m.close()
