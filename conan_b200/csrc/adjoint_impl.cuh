@@ -487,6 +487,11 @@ template <typename T, int R> struct Diff : DiffBase {
     // as forward leaves them and backward starts from (it ends at the initial
     // state)
     bool at_final = false;
+    // Calls that a caller captures run when the graph does, as often as it does,
+    // which the host does not see: the capture (0: none) that set at_final, and
+    // whether any call was captured.
+    unsigned long long final_capture = 0;
+    bool captured = false;
     // The launches of a pass between the caller's buffers, captured as graphs
     // from a handle's second pass on (a few microseconds of host time per
     // launch, and there are hundreds; building a graph pays from the second
@@ -589,6 +594,22 @@ template <typename T, int R> struct Diff : DiffBase {
         }
         CONAN_CUDA(cudaGraphLaunch(graphs[which], pm.st));
         return CONAN_OK;
+    }
+
+    // The caller's capture that the handle's stream takes part in (0: none).
+    int capture_id(unsigned long long *id) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        unsigned long long v = 0;
+        CONAN_CUDA(cudaStreamGetCaptureInfo(pm.st, &cs, &v));
+        *id = cs == cudaStreamCaptureStatusNone ? 0 : v;
+        captured = captured || *id;
+        return CONAN_OK;
+    }
+    // Whether this call (of capture `id`) finds the final state on the device:
+    // if the forward that left it there belongs to the same capture, or if
+    // neither it nor any other call of the handle was captured.
+    bool final_known(unsigned long long id) const {
+        return at_final && final_capture == id && (id || !captured);
     }
 
     // Orders the handle's stream after the caller's work. NULL is the legacy
@@ -697,6 +718,8 @@ template <typename T, int R> struct Diff : DiffBase {
 
     int forward(const void *noise, void *density, void *stream) override {
         CONAN_TRY(enter(stream));
+        unsigned long long cap = 0;
+        CONAN_TRY(capture_id(&cap));
         CONAN_TRY(take_noise(noise));
         CONAN_TRY(replay(G_STEPS, [&] { return forward_steps(); }));
         // the positions of the last deposit are the final ones: its density
@@ -705,6 +728,7 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_TRY(replay(G_LAST, [&] { return forward_last(); }));
         pm.mesh_holds = 2;
         at_final = have_forward = true;
+        final_capture = cap;
         return leave(stream);
     }
 
@@ -792,7 +816,9 @@ template <typename T, int R> struct Diff : DiffBase {
         if (!have_forward) return set_error(CONAN_ERR_STATE, "backward without a forward call");
         CONAN_TRY(enter(stream));
         cudaStream_t st = pm.st;
-        if (!at_final) CONAN_TRY(restore_final());  // a further gradient of the same forward
+        unsigned long long cap = 0;
+        CONAN_TRY(capture_id(&cap));
+        if (!final_known(cap)) CONAN_TRY(restore_final());  // a further gradient of the same forward
         at_final = false;
         // the density adjoint through the final deposit
         k_adj_deposit_grad<T, R><<<gp(), 256, 0, st>>>(pm.P, pm.mf, (const T *)gdens, pm.mass, db[0], db[1], db[2]);

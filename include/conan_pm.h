@@ -304,7 +304,9 @@ void conan_diff_destroy(conan_diff *h);
 /* Device pointers of the handle's precision (float or double):
  * noise N^dim, density_out N_f^dim. `stream` is a cudaStream_t (NULL: the
  * legacy default stream); the call is ordered after prior work on it, and
- * later work on it after the call (with NULL the call waits for its work). */
+ * later work on it after the call (with NULL the call waits for its work).
+ * Both calls may be captured from `stream` into graphs, together or apart; a
+ * backward call goes with the forward that ran last, in a graph or not. */
 int conan_diff_forward(conan_diff *h, const void *noise_dev, void *density_out_dev, void *stream);
 /* Gradient of a scalar loss w.r.t. the noise given its gradient w.r.t. the
  * final density of the last forward call. Further calls give the gradients of

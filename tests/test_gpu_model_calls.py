@@ -52,3 +52,65 @@ def test_a_further_gradient_of_one_forward(gpu, conan, prec, mbits, n, every):
     for gd, w in zip(losses[:2], want):
         assert torch.equal(torch.autograd.grad(delta, x, gd, retain_graph=True)[0], w)
     m.close()
+
+
+@pytest.mark.parametrize("prec,mbits,n,every", [("fp32", 6, 5, 2), ("fp64", 5, 3, 8)])
+def test_captured_calls(gpu, conan, prec, mbits, n, every):
+    from conan_b200.autograd import DiffPM
+    dt = torch.float32 if prec == "fp32" else torch.float64
+    m = DiffPM(dim=3, mbits=mbits, L_box=60.0, ns=-2.0, a0=0.05, da=0.08, n=n, checkpoint_every=every, precision=prec)
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    fields = [torch.randn(m.nnoise, device="cuda", dtype=dt, generator=gen) for _ in range(3)]
+    gd = torch.randn(m.ncells, device="cuda", dtype=dt, generator=gen) / m.ncells
+    noise, out, g = fields[0].clone(), torch.empty_like(gd), torch.empty_like(fields[0])
+    want = []
+    for f in fields:  # uncaptured, one forward each
+        noise.copy_(f)
+        m.forward_raw(noise, out)
+        m.backward_raw(gd, g)
+        want.append((out.clone(), g.clone()))
+
+    def check(i, density=True):
+        torch.cuda.synchronize()
+        assert torch.equal(g, want[i][1]) and (not density or torch.equal(out, want[i][0]))
+        g.zero_()
+        out.zero_()
+
+    graphs = []
+    for calls in ("fb", "f", "b"):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            if "f" in calls:
+                m.forward_raw(noise, out)
+            if "b" in calls:
+                m.backward_raw(gd, g)
+    both, fwd, bwd = graphs
+    g.zero_()
+    for i in (1, 2):  # one graph
+        noise.copy_(fields[i])
+        both.replay()
+        check(i)
+    noise.copy_(fields[0])  # a graph each, and a further gradient
+    fwd.replay()
+    bwd.replay()
+    check(0)
+    bwd.replay()
+    check(0, density=False)
+    noise.copy_(fields[1])  # a captured forward, uncaptured gradients
+    fwd.replay()
+    for density in (True, False):
+        m.backward_raw(gd, g)
+        check(1, density)
+    noise.copy_(fields[2])  # the other way, then a further gradient
+    m.forward_raw(noise, out)
+    bwd.replay()
+    check(2)
+    m.backward_raw(gd, g)
+    check(2, density=False)
+    noise.copy_(fields[0])  # and uncaptured again
+    m.forward_raw(noise, out)
+    m.backward_raw(gd, g)
+    check(0)
+    torch.cuda.synchronize()
+    del graphs, both, fwd, bwd
+    m.close()
