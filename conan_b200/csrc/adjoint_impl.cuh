@@ -585,7 +585,7 @@ template <typename T, int R> struct Diff : DiffBase {
                 return rc;
             }
             if (ce != cudaSuccess) return set_error(CONAN_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
-            const cudaError_t ie = cudaGraphInstantiate(&graphs[which], g, 0);
+            const cudaError_t ie = graph_instantiate(&graphs[which], g);
             cudaGraphDestroy(g);
             if (ie != cudaSuccess) {
                 graphs[which] = nullptr;
@@ -716,7 +716,16 @@ template <typename T, int R> struct Diff : DiffBase {
         return forward_last();
     }
 
+    // After a pass that failed the solver's host state says nothing about what
+    // its launches left pending.
+    int failed(int rc) {
+        if (rc != CONAN_OK) pm.stale = true;
+        return rc;
+    }
     int forward(const void *noise, void *density, void *stream) override {
+        return failed(forward_pass(noise, density, stream));
+    }
+    int forward_pass(const void *noise, void *density, void *stream) {
         CONAN_TRY(enter(stream));
         unsigned long long cap = 0;
         CONAN_TRY(capture_id(&cap));
@@ -814,6 +823,9 @@ template <typename T, int R> struct Diff : DiffBase {
 
     int backward(const void *gdens, void *gnoise, void *stream) override {
         if (!have_forward) return set_error(CONAN_ERR_STATE, "backward without a forward call");
+        return failed(backward_pass(gdens, gnoise, stream));
+    }
+    int backward_pass(const void *gdens, void *gnoise, void *stream) {
         CONAN_TRY(enter(stream));
         cudaStream_t st = pm.st;
         unsigned long long cap = 0;

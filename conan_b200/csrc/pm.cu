@@ -86,6 +86,13 @@ int device_guard(int dev) {
 
 // ------------------------------------------------------------------ PM --
 
+// cudaGraphInstantiate, with the failure that conan_selftest_fail_graph asks for.
+static thread_local int g_fail_graph = -1;
+static cudaError_t graph_instantiate(cudaGraphExec_t *x, cudaGraph_t g) {
+    if (g_fail_graph >= 0 && g_fail_graph-- == 0) return cudaErrorMemoryAllocation;
+    return cudaGraphInstantiate(x, g, 0);
+}
+
 template <typename T, int R> struct PM : PMBase {
     typedef typename Cplx<T>::type CT;
     typedef typename Pay<T>::elem PE;
@@ -490,8 +497,20 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
+    // A call failed between its launches: the host does not know which of them
+    // ran, so the ranks and accumulators may hold anything.
+    bool stale = false;
+
     // Particle positions were replaced: ranks and a fused deposit are stale.
     int positions_reset() {
+        if (stale) {
+            CONAN_CUDA(cudaMemsetAsync(count, 0, mf.cells * sizeof(uint32_t), st));
+            if (lacc) CONAN_CUDA(cudaMemsetAsync(lacc, 0, mf.cells * sizeof(unsigned long long), st));
+            if (dacc) CONAN_CUDA(cudaMemsetAsync(dacc, 0, mf.cells * sizeof(ulonglong2), st));
+            ranks_pending = lag_ready = stale = false;
+            mesh_holds = 0;
+            return CONAN_OK;
+        }
         if (ranks_pending) CONAN_CUDA(cudaMemsetAsync(count, 0, mf.cells * sizeof(uint32_t), st));
         ranks_pending = false;
         return drop_lag_deposit();
@@ -1310,7 +1329,7 @@ template <typename T, int R> struct PM : PMBase {
             if (cudaGraphExecUpdate(p->exec, g, &info) != cudaSuccess) {  // other launches: instantiate anew
                 cudaGetLastError();
                 cudaGraphExec_t fresh = nullptr;
-                ie = cudaGraphInstantiate(&fresh, g, 0);
+                ie = graph_instantiate(&fresh, g);
                 if (ie == cudaSuccess) {
                     cudaGraphExecDestroy(p->exec);
                     p->exec = fresh;
@@ -1322,7 +1341,7 @@ template <typename T, int R> struct PM : PMBase {
                 pieces.erase(pieces.begin());
             }
             cudaGraphExec_t fresh = nullptr;
-            ie = cudaGraphInstantiate(&fresh, g, 0);
+            ie = graph_instantiate(&fresh, g);
             if (ie == cudaSuccess) {
                 pieces.push_back({i1 - i0, first, last, fresh});
                 p = &pieces.back();
@@ -1335,13 +1354,19 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
-    // Steps [i0, i1) as graphs; returns after they have run.
+    // Steps [i0, i1) as graphs; returns after they have run. A piece that fails
+    // leaves the state and its scale factors as the pieces before it left them.
     int graph_segment(double &a, double da, unsigned i0, unsigned i1) {
         int rc = CONAN_OK;
         for (unsigned i = i0; i < i1 && rc == CONAN_OK;) {
             unsigned e = std::min(i1, i + PIECE);
             if (i1 - e < PIECE / 2) e = i1;  // no short last piece
+            const double ap = a_pos, am = a_mom;
             rc = graph_piece(a, da, i, e, i == i0, e == i1);
+            if (rc != CONAN_OK) {
+                a_pos = ap;
+                a_mom = am;
+            }
             i = e;
         }
         cudaError_t se = cudaStreamSynchronize(st);
@@ -1362,10 +1387,13 @@ template <typename T, int R> struct PM : PMBase {
                 seg_end = ((i / k) + 1) * k;
                 if (seg_end > n) seg_end = n;
             }
-            if (!prof.on && !debug_sync()) {
-                CONAN_TRY(graph_segment(a, da, i, seg_end));
-            } else {
-                CONAN_TRY(steps(a, da, i, seg_end));
+            const int rc = !prof.on && !debug_sync() ? graph_segment(a, da, i, seg_end) : steps(a, da, i, seg_end);
+            if (rc != CONAN_OK) {
+                const std::string msg = last_error();
+                stale = true;
+                positions_reset();
+                last_error() = msg;
+                return rc;
             }
             i = seg_end;
             if (cb) {
@@ -1603,6 +1631,11 @@ int conan_device_count(int *n) {
         c = 0;
     }
     *n = c;
+    return CONAN_OK;
+}
+
+int conan_selftest_fail_graph(int n) {
+    g_fail_graph = n;
     return CONAN_OK;
 }
 

@@ -63,6 +63,11 @@ int conan_device_count(int *n);
  * kernel. */
 int conan_selftest_bounded_wait(unsigned polls, void *stream);
 
+/* Makes the n-th (from 0) CUDA graph that this thread's coming run, forward and
+ * backward calls instantiate fail on the host as if memory had run out; a
+ * negative n takes that back. For tests of what a call leaves behind then. */
+int conan_selftest_fail_graph(int n);
+
 /* ------------------------------------------------------------------ ic -- */
 
 /* Options of the `ic` tool, src/ic/main.cc:15-65 (same names and meaning).

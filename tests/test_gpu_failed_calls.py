@@ -1,0 +1,98 @@
+"""What a call that failed on the host leaves behind: the next calls are right.
+The failures are made on the host (an error code in place of the call's own)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+# A run of 14 steps is four graphs of 4, 4, 4 and 2; the third is an update of
+# the second, so the graphs made anew are 0 (first), 1 (a middle one), 2 (last).
+# Lagrangian accumulator (FP32), two-word accumulator (FP64), sorted (FP64).
+@pytest.mark.parametrize("fail", [0, 1, 2])
+@pytest.mark.parametrize("prec,mode", [("fp32", None), ("fp64", None), ("fp64", "sorted")])
+def test_run_that_fails_between_its_graphs(gpu, conan, prec, mode, fail):
+    from conan_b200 import _lib as L
+    Nm, a0, da, n = 32, 0.05, 0.02, 14
+    phi = np.random.default_rng(1).normal(size=Nm ** 3) * 50
+
+    def handle():
+        g = conan.Gravity(3, Nm, 1, 100.0, precision=prec)
+        if mode:
+            g.deposit_mode = mode
+        return g
+
+    fresh = handle()
+    g = handle()
+    try:
+        L.lib().conan_selftest_fail_graph(fail)
+        with pytest.raises(conan.ConanError):
+            g.run(phi, a0, da, n)
+    finally:
+        L.lib().conan_selftest_fail_graph(-1)
+    # the state is that of the graphs before (up to the rounding of a kick and a
+    # drift in one kernel or two), and its density holds its mass once
+    a = a0
+    done = (0, 4, 12)[fail]
+    for _ in range(done):
+        a += da
+    X, P = g.state()
+    assert abs(g.density().mean()) < 1e-5
+    if done:
+        assert g.scale_factors() == pytest.approx((a, a - da / 2), abs=1e-12)
+        fresh.run(phi, a0, da, done)
+        fresh.drift(a, da)
+    else:
+        assert g.scale_factors() == (a0, a0 + da / 2)
+        fresh.init(phi, a0, a0 + da / 2)
+    Xf, Pf = fresh.state()
+    tol = 1e-5 if prec == "fp32" else 1e-11
+    assert np.max(np.abs(X - Xf)) < tol * 100 and np.max(np.abs(P - Pf)) < tol * np.max(np.abs(Pf))
+    # set anew, it runs as a fresh handle does
+    g.init(phi, a0, a0 + da / 2)
+    fresh.init(phi, a0, a0 + da / 2)
+    assert np.array_equal(g.density(), fresh.density())
+    g.run(phi, a0, da, n)
+    fresh.run(phi, a0, da, n)
+    for a, b in zip(g.state(), fresh.state()):
+        assert np.array_equal(a, b)
+    g.close()
+    fresh.close()
+
+
+# the model's second pass makes its graphs: the steps, the last step, the adjoint
+@pytest.mark.parametrize("fail", [0, 1, 2])
+@pytest.mark.parametrize("prec,mbits,plane", [("fp32", 5, "0"), ("fp64", 5, "0"), ("fp32", 8, "2")])
+def test_model_pass_that_fails(gpu, conan, monkeypatch, prec, mbits, plane, fail):
+    from conan_b200 import _lib as L
+    from conan_b200.autograd import DiffPM
+    monkeypatch.setenv("CONAN_PLANE_PASS", plane)
+    dt = torch.float32 if prec == "fp32" else torch.float64
+    m = DiffPM(dim=3, mbits=mbits, L_box=100.0, ns=-2.0, a0=0.05, da=0.05, n=3, checkpoint_every=2, precision=prec)
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    noise = torch.randn(m.nnoise, device="cuda", dtype=dt, generator=gen)
+    gd = torch.randn(m.ncells, device="cuda", dtype=dt, generator=gen) / m.ncells
+    ref, gref = torch.empty_like(gd), torch.empty_like(noise)
+    m.forward_raw(noise, ref)
+    m.backward_raw(gd, gref)
+    out, g = torch.empty_like(ref), torch.empty_like(gref)
+    try:
+        L.lib().conan_selftest_fail_graph(fail)
+        with pytest.raises(conan.ConanError):
+            m.forward_raw(noise, out)
+            m.backward_raw(gd, g)
+    finally:
+        L.lib().conan_selftest_fail_graph(-1)
+    if fail < 2:  # no forward to go with
+        with pytest.raises(conan.ConanError):
+            m.backward_raw(gd, g)
+    else:
+        m.backward_raw(gd, g)
+        assert torch.equal(g, gref)
+    for _ in range(2):
+        m.forward_raw(noise, out)
+        m.backward_raw(gd, g)
+        assert torch.equal(out, ref) and torch.equal(g, gref)
+    m.close()
