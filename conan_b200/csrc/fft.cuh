@@ -15,39 +15,34 @@ struct FFTPair {
     bool dbl = false;
 
     int create(const Mesh &m, bool is_double, int batch) {
-        dbl = is_double;
-        int n[3];
-        for (int i = 0; i < m.R; ++i) n[i] = m.n;  // cubic: slowest..fastest all n
-        long long real_dist = 1LL << m.cshift, cplx_dist = (long long)m.mspec;
-        size_t w1 = 0, w2 = 0;
-        CONAN_CUFFT(cufftCreate(&r2c));
-        CONAN_CUFFT(cufftCreate(&c2r));
-        CONAN_CUFFT(cufftSetAutoAllocation(r2c, 0));
-        CONAN_CUFFT(cufftSetAutoAllocation(c2r, 0));
-        CONAN_CUFFT(cufftMakePlanMany(r2c, m.R, n, nullptr, 1, (int)real_dist, nullptr, 1,
-                                      (int)cplx_dist, dbl ? CUFFT_D2Z : CUFFT_R2C, batch, &w1));
-        CONAN_CUFFT(cufftMakePlanMany(c2r, m.R, n, nullptr, 1, (int)cplx_dist, nullptr, 1,
-                                      (int)real_dist, dbl ? CUFFT_Z2D : CUFFT_C2R, batch, &w2));
-        work_bytes = w1 > w2 ? w1 : w2;
-        return CONAN_OK;
+        return make(m.R, m.n, 1LL << m.cshift, (long long)m.mspec, is_double, batch);
     }
     // The same half-spectrum layout with the slowest axis left in real space: 2D
     // transforms of every z plane of 3D meshes, 1D ones of every row of 2D ones.
     int create_planes(const Mesh &m, bool is_double, int batch) {
+        const long long rows = m.R == 3 ? m.n : 1;  // per plane
+        return make(m.R - 1, m.n, rows * m.n, rows * m.nh, is_double, batch * m.n);
+    }
+    // `batch` pairs of rank-dimensional transforms of n cells per side, real_dist
+    // and cplx_dist values apart. A pair that cannot be made whole has no
+    // handles, so that they always stand for plans.
+    int make(int rank, int side, long long real_dist, long long cplx_dist, bool is_double, int batch) {
+        const int rc = plan(rank, side, real_dist, cplx_dist, is_double, batch);
+        if (rc != CONAN_OK) destroy();
+        return rc;
+    }
+    int plan(int rank, int side, long long real_dist, long long cplx_dist, bool is_double, int batch) {
         dbl = is_double;
-        int n[2] = {m.n, m.n};
-        const int rank = m.R - 1;
-        long long real_dist = rank == 2 ? (long long)m.n * m.n : m.n, cplx_dist = rank == 2 ? (long long)m.n * m.nh : m.nh;
-        const int planes = batch * m.n;
+        int n[3] = {side, side, side};
         size_t w1 = 0, w2 = 0;
         CONAN_CUFFT(cufftCreate(&r2c));
         CONAN_CUFFT(cufftCreate(&c2r));
         CONAN_CUFFT(cufftSetAutoAllocation(r2c, 0));
         CONAN_CUFFT(cufftSetAutoAllocation(c2r, 0));
         CONAN_CUFFT(cufftMakePlanMany(r2c, rank, n, nullptr, 1, (int)real_dist, nullptr, 1, (int)cplx_dist,
-                                      dbl ? CUFFT_D2Z : CUFFT_R2C, planes, &w1));
+                                      dbl ? CUFFT_D2Z : CUFFT_R2C, batch, &w1));
         CONAN_CUFFT(cufftMakePlanMany(c2r, rank, n, nullptr, 1, (int)cplx_dist, nullptr, 1, (int)real_dist,
-                                      dbl ? CUFFT_Z2D : CUFFT_C2R, planes, &w2));
+                                      dbl ? CUFFT_Z2D : CUFFT_C2R, batch, &w2));
         work_bytes = w1 > w2 ? w1 : w2;
         return CONAN_OK;
     }

@@ -214,7 +214,7 @@ int plan_take(const Mesh &m, bool is_double, FFTPair *fft) {
 }
 
 void plan_return(const Mesh &m, bool is_double, FFTPair *fft) {
-    if (!fft->r2c || !fft->c2r) {  // a pair that was not made whole
+    if (!fft->r2c || !fft->c2r) {  // a pair that was not made
         fft->destroy();
         return;
     }
