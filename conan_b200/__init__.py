@@ -20,11 +20,12 @@ from .pm import (  # noqa: E402
     compute_potential,
     generate_random_field,
     ic_params,
+    release_caches,
     white_noise,
 )
 from .conanfile import ConanFile  # noqa: E402
 
 __all__ = [
     "ConanError", "ConanFile", "Cosmology", "FoF", "Gravity", "LeapFrog", "cic", "compute_displacement",
-    "compute_potential", "fof", "generate_random_field", "ic_params", "white_noise",
+    "compute_potential", "fof", "generate_random_field", "ic_params", "release_caches", "white_noise",
 ]

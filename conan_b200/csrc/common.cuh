@@ -71,6 +71,25 @@ template <typename K> bool raise_dyn_smem(K kern, size_t bytes) {
     return true;
 }
 
+// Gives back what calls without a handle keep idle for the next ones (hostio.cu).
+int release_caches();
+
+// An allocation (of device memory, or of what takes some) that is tried once
+// more after release_caches where the device is full. (The present driver takes
+// a pool's idle memory for cudaMalloc by itself; this does not rely on it.)
+template <typename F> cudaError_t alloc_retry(F f) {
+    cudaError_t e = f();
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        release_caches();
+        e = f();
+    }
+    return e;
+}
+template <typename U> cudaError_t device_alloc(U **p, size_t bytes) {
+    return alloc_retry([&] { return cudaMalloc((void **)p, bytes); });
+}
+
 inline bool is_pow2(long long n) { return n > 0 && (n & (n - 1)) == 0; }
 inline int ilog2(long long n) {
     int s = 0;

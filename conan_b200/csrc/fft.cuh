@@ -27,24 +27,34 @@ struct FFTPair {
     // and cplx_dist values apart. A pair that cannot be made whole has no
     // handles, so that they always stand for plans.
     int make(int rank, int side, long long real_dist, long long cplx_dist, bool is_double, int batch) {
-        const int rc = plan(rank, side, real_dist, cplx_dist, is_double, batch);
-        if (rc != CONAN_OK) destroy();
-        return rc;
-    }
-    int plan(int rank, int side, long long real_dist, long long cplx_dist, bool is_double, int batch) {
         dbl = is_double;
+        cufftResult r = plan(rank, side, real_dist, cplx_dist, batch);
+        if (r == CUFFT_ALLOC_FAILED) {  // see alloc_retry
+            destroy();
+            cudaGetLastError();
+            release_caches();
+            r = plan(rank, side, real_dist, cplx_dist, batch);
+        }
+        if (r == CUFFT_SUCCESS) return CONAN_OK;
+        destroy();
+        return set_error(CONAN_ERR_CUDA, "%d FFT plans of dimension %d and %d cells failed: cufft error %d", batch, rank,
+                         side, (int)r);
+    }
+    cufftResult plan(int rank, int side, long long real_dist, long long cplx_dist, int batch) {
         int n[3] = {side, side, side};
         size_t w1 = 0, w2 = 0;
-        CONAN_CUFFT(cufftCreate(&r2c));
-        CONAN_CUFFT(cufftCreate(&c2r));
-        CONAN_CUFFT(cufftSetAutoAllocation(r2c, 0));
-        CONAN_CUFFT(cufftSetAutoAllocation(c2r, 0));
-        CONAN_CUFFT(cufftMakePlanMany(r2c, rank, n, nullptr, 1, (int)real_dist, nullptr, 1, (int)cplx_dist,
-                                      dbl ? CUFFT_D2Z : CUFFT_R2C, batch, &w1));
-        CONAN_CUFFT(cufftMakePlanMany(c2r, rank, n, nullptr, 1, (int)cplx_dist, nullptr, 1, (int)real_dist,
-                                      dbl ? CUFFT_Z2D : CUFFT_C2R, batch, &w2));
+        cufftResult r = cufftCreate(&r2c);
+        if (r == CUFFT_SUCCESS) r = cufftCreate(&c2r);
+        if (r == CUFFT_SUCCESS) r = cufftSetAutoAllocation(r2c, 0);
+        if (r == CUFFT_SUCCESS) r = cufftSetAutoAllocation(c2r, 0);
+        if (r == CUFFT_SUCCESS)
+            r = cufftMakePlanMany(r2c, rank, n, nullptr, 1, (int)real_dist, nullptr, 1, (int)cplx_dist,
+                                  dbl ? CUFFT_D2Z : CUFFT_R2C, batch, &w1);
+        if (r == CUFFT_SUCCESS)
+            r = cufftMakePlanMany(c2r, rank, n, nullptr, 1, (int)cplx_dist, nullptr, 1, (int)real_dist,
+                                  dbl ? CUFFT_Z2D : CUFFT_C2R, batch, &w2);
         work_bytes = w1 > w2 ? w1 : w2;
-        return CONAN_OK;
+        return r;
     }
     int bind(void *work, cudaStream_t s) {
         CONAN_CUFFT(cufftSetWorkArea(r2c, work));

@@ -562,25 +562,25 @@ struct FofEngine {
         const size_t tiles = radix_tiles(n), m = 256 * tiles;
         const size_t nb = (std::max(std::max(m, rows), n) + SCAN_CHUNK - 1) / SCAN_CHUNK;
         CONAN_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        CONAN_CUDA(cudaMalloc(&X, n * R * sizeof(double)));
-        CONAN_CUDA(cudaMalloc(&S, n * R * sizeof(double)));
+        CONAN_CUDA(device_alloc(&X, n * R * sizeof(double)));
+        CONAN_CUDA(device_alloc(&S, n * R * sizeof(double)));
         for (int b = 0; b < 2; ++b) {
-            CONAN_CUDA(cudaMalloc(&keys[b], n * sizeof(uint64_t)));
-            CONAN_CUDA(cudaMalloc(&vals[b], n * sizeof(uint32_t)));
+            CONAN_CUDA(device_alloc(&keys[b], n * sizeof(uint64_t)));
+            CONAN_CUDA(device_alloc(&vals[b], n * sizeof(uint32_t)));
         }
-        CONAN_CUDA(cudaMalloc(&par, n * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&flag, n * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&gnum, (n + 1) * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&rowcount, rows * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&rowoff, (rows + 1) * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&bh, m * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&boff, (m + 1) * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&bsum, nb * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&tags, n * sizeof(unsigned long long)));
-        CONAN_CUDA(cudaMalloc(&err, sizeof(int)));
+        CONAN_CUDA(device_alloc(&par, n * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&flag, n * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&gnum, (n + 1) * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&rowcount, rows * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&rowoff, (rows + 1) * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&bh, m * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&boff, (m + 1) * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&bsum, nb * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&tags, n * sizeof(unsigned long long)));
+        CONAN_CUDA(device_alloc(&err, sizeof(int)));
         CONAN_CUDA(cudaMallocHost(&ngroups_h, 2 * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&bigrows, std::min(rows, n / 33 + 1) * sizeof(uint32_t)));
-        CONAN_CUDA(cudaMalloc(&nbig, 2 * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&bigrows, std::min(rows, n / 33 + 1) * sizeof(uint32_t)));
+        CONAN_CUDA(device_alloc(&nbig, 2 * sizeof(uint32_t)));
         CONAN_CUDA(cudaMallocHost(&nbig_h, 2 * sizeof(uint32_t)));
         int sms = 0;
         CONAN_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));

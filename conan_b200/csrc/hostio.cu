@@ -184,13 +184,7 @@ cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t st) {
         pool = c.pool[dev];
     }
     if (!pool) return cudaErrorInvalidDevice;
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st);
-    if (e == cudaErrorMemoryAllocation) {  // idle memory in other sizes
-        cudaGetLastError();
-        cudaMemPoolTrimTo(pool, 0);
-        e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st);
-    }
-    return e;
+    return alloc_retry([&] { return cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st); });
 }
 void pool_free(void *p, cudaStream_t st) {
     if (p) cudaFreeAsync(p, st);

@@ -40,6 +40,4 @@ void pool_free(void *p, cudaStream_t st);
 int plan_take(const Mesh &m, bool is_double, FFTPair *fft);
 void plan_return(const Mesh &m, bool is_double, FFTPair *fft);
 
-int release_caches();
-
 }  // namespace conan

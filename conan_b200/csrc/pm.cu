@@ -90,7 +90,7 @@ int device_guard(int dev) {
 static thread_local int g_fail_graph = -1;
 static cudaError_t graph_instantiate(cudaGraphExec_t *x, cudaGraph_t g) {
     if (g_fail_graph >= 0 && g_fail_graph-- == 0) return cudaErrorMemoryAllocation;
-    return cudaGraphInstantiate(x, g, 0);
+    return alloc_retry([&] { return cudaGraphInstantiate(x, g, 0); });
 }
 
 template <typename T, int R> struct PM : PMBase {
@@ -145,12 +145,7 @@ template <typename T, int R> struct PM : PMBase {
         void *q = nullptr;
         size_t b = n * sizeof(U);
         if (b == 0) b = 16;
-        cudaError_t e = cudaMalloc(&q, b);
-        if (e == cudaErrorMemoryAllocation) {  // what the handle-less calls keep idle may be enough
-            cudaGetLastError();
-            release_caches();
-            e = cudaMalloc(&q, b);
-        }
+        const cudaError_t e = device_alloc(&q, b);
         if (e != cudaSuccess) {
             cudaGetLastError();
             return set_error(CONAN_ERR_ALLOC, "cudaMalloc of %zu bytes failed: %s", b, cudaGetErrorString(e));
@@ -1038,7 +1033,14 @@ template <typename T, int R> struct PM : PMBase {
         tuned.clear();
         const double apos = a_pos, amom = a_mom;
         std::vector<T *> save(2 * R, nullptr);
-        for (auto &b : save) CONAN_CUDA(cudaMalloc(&b, np * sizeof(T)));
+        for (auto &b : save) {
+            const cudaError_t e = device_alloc(&b, np * sizeof(T));
+            if (e == cudaSuccess) continue;
+            cudaGetLastError();
+            for (auto c : save) cudaFree(c);
+            return set_error(CONAN_ERR_ALLOC, "no memory for the autotuner's copy of the state: %s",
+                             cudaGetErrorString(e));
+        }
         for (int k = 0; k < R; ++k) {
             CONAN_CUDA(cudaMemcpyAsync(save[k], P.d[k], np * sizeof(T), cudaMemcpyDeviceToDevice, st));
             CONAN_CUDA(cudaMemcpyAsync(save[R + k], P.p[k], np * sizeof(T), cudaMemcpyDeviceToDevice, st));
@@ -1529,8 +1531,9 @@ int spectrum_bins(const typename Cplx<T>::type *spec, const Mesh &m, double L, i
     size_t sh = (size_t)(threads / 32) * 3 * nbins * sizeof(double);
     if (sh > 200 * 1024) return set_error(CONAN_ERR_ARG, "too many bins (%d)", nbins);
     double *part = nullptr, *out = nullptr;
-    CONAN_CUDA(cudaMallocAsync((void **)&part, (size_t)nblocks * 3 * nbins * sizeof(double), st));
-    CONAN_CUDA(cudaMallocAsync((void **)&out, 3 * (size_t)nbins * sizeof(double), st));
+    CONAN_CUDA(alloc_retry(
+        [&] { return cudaMallocAsync((void **)&part, (size_t)nblocks * 3 * nbins * sizeof(double), st); }));
+    CONAN_CUDA(alloc_retry([&] { return cudaMallocAsync((void **)&out, 3 * (size_t)nbins * sizeof(double), st); }));
     if (sh > 48 * 1024)
         CONAN_CUDA(cudaFuncSetAttribute(k_pk_partial<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
     k_pk_partial<T><<<nblocks, threads, sh, st>>>(spec, m, nbins, part);

@@ -112,6 +112,13 @@ def cic(X: np.ndarray, dim: int, n_mass: int, L_box: float, f: int = 2, sub_samp
     return out
 
 
+def release_caches():
+    """Gives back the staging memory, device memory and FFT plans that calls on
+    host arrays (ic, cic, fof, states) keep for the next ones, e.g. before
+    another library needs the device memory (conan_release_caches)."""
+    L.check(L.lib().conan_release_caches())
+
+
 def _fof_params(dim, n, L_box, linking_length, device):
     p = L.FofParams()
     p.dim, p.n_particles, p.size, p.linking_length, p.device = dim, n, float(L_box), float(linking_length), device

@@ -111,7 +111,8 @@ int conan_ic_displacement(const conan_ic_params *p, const double *potential, dou
 /* Calls that take host arrays keep a bounded cache for the next ones: per
  * device at most 16 MiB of page-locked staging memory and 512 MiB of device
  * memory, and four pairs of FFT plans. This gives all of it back (what calls
- * under way on other threads hold stays theirs). No reference counterpart. */
+ * under way on other threads hold stays theirs); calls of this library that
+ * find the device full do so by themselves. No reference counterpart. */
 int conan_release_caches(void);
 
 /* ----------------------------------------------------------------- cic -- */

@@ -1,6 +1,7 @@
 """The cache of idle FFT plans, on the host: the library's cuFFT calls go to a
 stand-in that counts plans and fails where it is told to. A pair that could not
-be planned is destroyed and never handed to a later call."""
+be planned is destroyed and never handed to a later call; one that finds no
+memory is planned again once the idle pairs are given back."""
 import os
 import subprocess
 import sys
@@ -54,6 +55,16 @@ for at in (0, 1):  # the forward, then the inverse plan cannot be made
     assert take(r) == 0 and (r.r2c, r.c2r) == (var("handles").value - 1, var("handles").value)
     give(r)
     assert lib.conan_release_caches() == 0 and var("live").value == 0
+# no memory (CUFFT_ALLOC_FAILED): the idle pair goes, and planning succeeds
+p = Pair()
+assert take(p) == 0
+give(p)
+m.n, m.shift, m.cshift = 64, 6, 18
+var("calls").value, var("fail_at").value, var("fail_code").value = 0, 1, 2
+q = Pair()
+assert take(q) == 0 and planned[q.r2c] and planned[q.c2r] and not planned[p.r2c] and var("live").value == 2
+give(q)
+assert lib.conan_release_caches() == 0 and var("live").value == 0
 """
 
 
