@@ -307,7 +307,7 @@ template <typename T, int R> struct Ens : EnsBase {
         auto &c = cls[where[member].first];
         auto &pm = c.d->pm;
         CONAN_TRY(pm.deposit());
-        CONAN_TRY(pm.fft.forward(pm.mesh, pm.spec));
+        CONAN_TRY(pm.full_spectrum());
         Mesh m1 = make_mesh(R, pm.mf.n, 1);
         CONAN_TRY(spectrum_bins<T>(pm.spec + (size_t)where[member].second * m1.mspec, m1, c.L, nbins, k, Pk, cnt,
                                    pm.st, nullptr));

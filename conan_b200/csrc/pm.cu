@@ -137,9 +137,9 @@ template <typename T, int R> struct PM : PMBase {
     static constexpr size_t STAGE_MAX = (size_t)1 << 24;  // doubles per chunk (128 MiB)
     void *work = nullptr;
     FFTPair fft;
-    // FP32 3D FD4 meshes of 64..1024 cells per side: the Poisson solve as 2D
-    // transforms of the z planes around the shared-memory z pass (fft_z.cuh)
-    // (FP64, 2D of 64..1024 and 3D of 64..512 cells per side: fft_line64.cuh)
+    // FD4 meshes whose Poisson solve is the transforms of all axes but the last
+    // (fft2) around a shared-memory pass along that one: FP32 3D of 64..1024 cells
+    // per side (fft_z.cuh), FP64 2D of 64..1024 and 3D of 64..512 (fft_line64.cuh)
     FFTPair fft2;
     CT *ztw = nullptr;  // exp(-2 pi i k / n), k < n
     bool zpass = false;
@@ -238,14 +238,14 @@ template <typename T, int R> struct PM : PMBase {
             CONAN_CUDA(cudaMemsetAsync(dacc, 0, mf.cells * sizeof(ulonglong2), st));
             dep_variant = DEP_DIRECT;
         }
-        CONAN_TRY(fft.create(mf, sizeof(T) == 8, batch));
-        size_t wbytes = fft.work_bytes;
         const bool split = sizeof(T) == 4 ? R == 3 && mf.n <= 1024 : (R == 3 && mf.n <= 512) || (R == 2 && mf.n <= 1024);
-        if (split && p.gradient == CONAN_GRAD_FD4 && mf.n >= 64) {
+        zpass = split && p.gradient == CONAN_GRAD_FD4 && mf.n >= 64;
+        if (!zpass || sizeof(T) == 4) CONAN_TRY(fft.create(mf, sizeof(T) == 8, batch));
+        size_t wbytes = fft.work_bytes;
+        if (zpass) {
             CONAN_TRY(fft2.create_planes(mf, sizeof(T) == 8, batch));
             CONAN_TRY(zpass_setup());
             wbytes = std::max(wbytes, fft2.work_bytes);
-            zpass = true;
             if (lacc) CONAN_TRY(plane_setup());
         }
         // CONAN_GRAD_KERNEL: cell or zm picks the gradient-mesh kernel at
@@ -253,9 +253,27 @@ template <typename T, int R> struct PM : PMBase {
         grad_zm = mf.cells > ((size_t)1 << 21);
         if (const char *gk = getenv("CONAN_GRAD_KERNEL")) grad_zm = !strcmp(gk, "zm");
         CONAN_TRY(alloc((char **)&work, wbytes));
-        CONAN_TRY(fft.bind(work, st));
+        if (fft.r2c) CONAN_TRY(fft.bind(work, st));
         if (zpass) CONAN_TRY(fft2.bind(work, st));
         CONAN_CUDA(cudaStreamSynchronize(st));
+        return CONAN_OK;
+    }
+
+    // Half spectrum of the density in mesh by the full transforms, for the power
+    // spectrum. FP64 handles that solve around the line pass make those
+    // transforms' plans at the first one (creation with both pairs: 64^2 cells 1.6
+    // ms against 1.0, 256^2 3.4 against 2.7, 64^3 6.8 against 6.0); their work
+    // area is the gradient mesh (32 bytes per cell), which only lives from a solve
+    // to its kick.
+    int full_spectrum() {
+        if (!fft.r2c) {
+            CONAN_TRY(fft.create(mf, sizeof(T) == 8, mf.batch));
+            void *w = grad;
+            if (fft.work_bytes > mf.cells * sizeof(G4<T>)) CONAN_TRY(alloc((char **)&w, fft.work_bytes));
+            CONAN_TRY(fft.bind(w, st));
+        }
+        CONAN_TIMED(prof, "fft_r2c", st, CONAN_TRY(fft.forward(mesh, spec)));
+        mesh_holds = 1;
         return CONAN_OK;
     }
 
@@ -1489,8 +1507,7 @@ template <typename T, int R> struct PM : PMBase {
     int power_spectrum(int nbins, double *k, double *Pk, double *cnt) override {
         if (nbins < 1) return set_error(CONAN_ERR_ARG, "nbins must be positive");
         CONAN_TRY(deposit());
-        CONAN_TIMED(prof, "fft_r2c", st, CONAN_TRY(fft.forward(mesh, spec)));
-        mesh_holds = 1;
+        CONAN_TRY(full_spectrum());
         CONAN_TRY(spectrum_bins<T>(spec, mf, prm.size, nbins, k, Pk, cnt, st, this));
         return check_err();
     }
