@@ -121,14 +121,18 @@ template <int R> int choose_window(int n, int f, LagWin *w, size_t *smem) {
     // the small tiles first: always in 3D (these kernels read global memory
     // without staging; 128^3 44 -> 36 us, 64^3 9.1 -> 7.6), in 2D where they
     // are one wave (512^2: 64 x 32 tiles 14.4 us per call against 15.5)
-    int v = (R == 3 || lag_small<R>((size_t)1 << (R * ilog2(n)))) && window_of<R, LAG_SMALL>(n, f, false, w, smem)
-                ? LAG_SMALL
-            : window_of<R, 0>(n, f, false, w, smem) ? 0 : window_of<R, 1>(n, f, false, w, smem) ? 1
+    int v = -1;
+    double per = 0;
+    if constexpr (R > 1)
+        if ((R == 3 || lag_small<R>((size_t)1 << (R * ilog2(n)))) && window_of<R, LAG_SMALL>(n, f, false, w, smem)) {
+            v = LAG_SMALL;
+            per = tile_particles<R, LAG_SMALL>();
+        }
+    if (v < 0) {
+        v = window_of<R, 0>(n, f, false, w, smem) ? 0 : window_of<R, 1>(n, f, false, w, smem) ? 1
             : window_of<R, 2>(n, f, false, w, smem) ? 2 : -1;
-    const double per = v == 0   ? tile_particles<R, 0>()
-                       : v == 1 ? tile_particles<R, 1>()
-                       : v == 2 ? tile_particles<R, 2>()
-                                : tile_particles<R, LAG_SMALL>();
+        per = v == 0 ? tile_particles<R, 0>() : v == 1 ? tile_particles<R, 1>() : tile_particles<R, 2>();
+    }
     if (v < 0 || (double)w->cells > LAG_WINDOW_CELLS_PER_PARTICLE * per)
         v = window_of<R, 0>(n, f, true, w, smem) ? 0 : window_of<R, 1>(n, f, true, w, smem) ? 1
             : window_of<R, 2>(n, f, true, w, smem) ? 2 : -1;

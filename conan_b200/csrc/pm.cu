@@ -217,8 +217,8 @@ template <typename T, int R> struct PM : PMBase {
         CONAN_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
         CONAN_CUDA(cudaMemsetAsync(count, 0, mf.cells * sizeof(uint32_t), st));
         dep_variant = dep_default();
-        bool lag = sizeof(T) == 4 && ((lag_small<R>(np) && lag_try<LAG_SMALL>()) || lag_try<0>() || lag_try<1>() ||
-                                  lag_try<2>());
+        bool lag = sizeof(T) == 4 &&
+                   ((lag_small<R>(np) && lag_set(LAG_SMALL, false)) || lag_try<0>() || lag_try<1>() || lag_try<2>());
         // On fine meshes (f >= 2) a window that fits shared memory only fits
         // a small tile and holds many cells per particle, each of which gets
         // about one corner: clearing and flushing it costs more than the
@@ -340,11 +340,26 @@ template <typename T, int R> struct PM : PMBase {
 
     bool lag_on() const { return sizeof(T) == 4 && dep_variant == DEP_LAG && lag_v >= 0 && lacc; }
 
+    // f(V) with lattice-tile variant v as a compile-time constant.
+    template <typename F> static int lag_call(int v, F f) {
+        if (v == 0) return f(std::integral_constant<int, 0>{});
+        if (v == 1) return f(std::integral_constant<int, 1>{});
+        if (v == 2) return f(std::integral_constant<int, 2>{});
+        if constexpr (R > 1)
+            if (v == LAG_SMALL) return f(std::integral_constant<int, LAG_SMALL>{});
+        return set_error(CONAN_ERR_STATE, "no lattice tile %d", v);
+    }
+
     template <int V> static constexpr double lag_tile_particles() {
         return (double)LagTile<R, V>::LX * LagTile<R, V>::LY * LagTile<R, V>::LZ;
     }
     double lag_particles() const {
-        return lag_v == 0 ? lag_tile_particles<0>() : lag_v == 1 ? lag_tile_particles<1>() : lag_v == 2 ? lag_tile_particles<2>() : lag_tile_particles<3>();
+        double n = 0;
+        lag_call(lag_v, [&](auto v) {
+            n = lag_tile_particles<decltype(v)::value>();
+            return CONAN_OK;
+        });
+        return n;
     }
 
     // direct: a window of two cells per axis, so that (nearly) every corner
@@ -396,10 +411,7 @@ template <typename T, int R> struct PM : PMBase {
         if constexpr (sizeof(T) == 4 && R == 3) {
             const char *off = getenv("CONAN_NO_TMA");
             if (off && *off && *off != '0') return CONAN_OK;
-            if (lag_v == 0) return tma_setup_v<0>();
-            if (lag_v == 1) return tma_setup_v<1>();
-            if (lag_v == 2) return tma_setup_v<2>();
-            if (lag_v == 3) return tma_setup_v<3>();
+            if (lag_v >= 0) return lag_call(lag_v, [&](auto v) { return tma_setup_v<decltype(v)::value>(); });
         }
         return CONAN_OK;
     }
@@ -474,7 +486,10 @@ template <typename T, int R> struct PM : PMBase {
         return CONAN_OK;
     }
 
-    template <int V> int launch_gkd_lag(const GKD &c, const char *name) {
+    int launch_gkd_lag(const GKD &c, const char *name) {
+        return lag_call(lag_v, [&](auto v) { return launch_gkd_lag_v<decltype(v)::value>(c, name); });
+    }
+    template <int V> int launch_gkd_lag_v(const GKD &c, const char *name) {
         if constexpr (sizeof(T) == 4) {
             typedef LagTile<R, V> L;
             size_t tiles = (size_t)(mm.n / L::LX) * (R >= 2 ? mm.n / L::LY : 1) * (R == 3 ? mm.n / L::LZ : 1) *
@@ -555,14 +570,10 @@ template <typename T, int R> struct PM : PMBase {
         if (!lag_ready) {
             if (tma_ok && !pers_ok) {  // the staged tiles, neither kick nor drift
                 const GKD c{0, 0, 0, 0, 0, 0};
-                if (lag_v == 0) CONAN_TRY(launch_gkd_lag<0>(c, "deposit"));
-                else if (lag_v == 1) CONAN_TRY(launch_gkd_lag<1>(c, "deposit"));
-                else if (lag_v == 2) CONAN_TRY(launch_gkd_lag<2>(c, "deposit"));
-                else CONAN_TRY(launch_gkd_lag<3>(c, "deposit"));
-            } else if (lag_v == 0) CONAN_TRY(launch_lag<0>());
-            else if (lag_v == 1) CONAN_TRY(launch_lag<1>());
-            else if (lag_v == 2) CONAN_TRY(launch_lag<2>());
-            else CONAN_TRY(launch_lag<3>());
+                CONAN_TRY(launch_gkd_lag(c, "deposit"));
+            } else {
+                CONAN_TRY(lag_call(lag_v, [&](auto v) { return launch_lag<decltype(v)::value>(); }));
+            }
         }
         lag_ready = false;
         return CONAN_OK;
@@ -1029,8 +1040,12 @@ template <typename T, int R> struct PM : PMBase {
         return mf.n >= D::TX && mf.n >= D::TY && mf.n >= D::TZ;
     }
     bool lag_set(int v, bool direct) {
-        return v == 0 ? lag_try<0>(direct) : v == 1 ? lag_try<1>(direct) : v == 2 ? lag_try<2>(direct)
-                                                                                 : lag_try<LAG_SMALL>(direct);
+        bool ok = false;
+        lag_call(v, [&](auto w) {
+            ok = lag_try<decltype(w)::value>(direct);
+            return CONAN_OK;
+        });
+        return ok;
     }
     int dep_apply(const DepCand &c) {
         CONAN_TRY(drop_lag_deposit());
@@ -1119,7 +1134,7 @@ template <typename T, int R> struct PM : PMBase {
             if (R == 3) tile[0] = "32x8x8", tile[1] = "16x8x8", tile[2] = "8x8x8", tile[3] = "16x8x4";
             if (R == 2) tile[0] = "64x32", tile[1] = "32x16", tile[2] = "16x16", tile[3] = "16x16 / 256 threads";
             if (R == 1) tile[0] = "2048", tile[1] = "512", tile[2] = "128";
-            for (int v = 0; v < (lag_small<R>(np) ? 4 : 3); ++v)
+            for (int v = 0; v < (lag_small<R>(np) ? LAG_SMALL + 1 : LAG_SMALL); ++v)
                 if (lag_set(v, false)) cands.push_back({1, v, std::string("lagrangian window, tile ") + tile[v]});
             if (R == 3)
                 for (int v = 0; v < 2; ++v)
@@ -1252,11 +1267,7 @@ template <typename T, int R> struct PM : PMBase {
         GKD c{ck, cd, kick ? 1 : 0, drift ? 1 : 0, rank_after ? 1 : 0, prm.periodic_gather ? 1 : 0};
         const char *name = kick ? (drift ? "gather_kick_drift" : "gather_kick") : "drift";
         if (fuse) {
-            const char *fname = kick ? "gather_kick_drift_deposit" : "drift_deposit";
-            if (lag_v == 0) CONAN_TRY(launch_gkd_lag<0>(c, fname));
-            else if (lag_v == 1) CONAN_TRY(launch_gkd_lag<1>(c, fname));
-            else if (lag_v == 2) CONAN_TRY(launch_gkd_lag<2>(c, fname));
-            else CONAN_TRY(launch_gkd_lag<3>(c, fname));
+            CONAN_TRY(launch_gkd_lag(c, kick ? "gather_kick_drift_deposit" : "drift_deposit"));
             lag_ready = true;
             return CONAN_OK;
         }
@@ -1264,11 +1275,7 @@ template <typename T, int R> struct PM : PMBase {
         // tiles instead of the thread-per-particle kernel
         if (kick && !drift && !rank_after && lag_on() && prm.gradient == CONAN_GRAD_FD4) {
             c.deposit = 0;
-            if (lag_v == 0) CONAN_TRY(launch_gkd_lag<0>(c, name));
-            else if (lag_v == 1) CONAN_TRY(launch_gkd_lag<1>(c, name));
-            else if (lag_v == 2) CONAN_TRY(launch_gkd_lag<2>(c, name));
-            else CONAN_TRY(launch_gkd_lag<3>(c, name));
-            return CONAN_OK;
+            return launch_gkd_lag(c, name);
         }
         ulonglong2 *const da = direct ? dacc : nullptr;
         if (prm.gradient == CONAN_GRAD_SPECTRAL)

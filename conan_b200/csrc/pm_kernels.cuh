@@ -854,8 +854,8 @@ struct LagWin {
 };
 
 // Lattice tile (LX x LY x LZ particles), threads and window margin M (cells
-// beyond the tile's own f*L cells, split over both sides) of variant V.
-constexpr int LAG_VARIANTS = 4;
+// beyond the tile's own f*L cells, split over both sides) of variant V: 0 to 2
+// in every dimension, LAG_SMALL in 2D and 3D.
 // 32-bit planes of a window cell: 2 keeps the carry in shared memory, 1
 // sends it to the accumulator mesh (a carry needs over 2^9 particles' weight
 // in one cell of one tile: rare). A compile-time tunable; one plane leaves
@@ -883,7 +883,6 @@ template <> struct LagTile<3, 2> { static constexpr int LX = 8, LY = 8, LZ = 8, 
 constexpr int LAG_SMALL = 3;
 template <> struct LagTile<3, 3> { static constexpr int LX = 16, LY = 8, LZ = 4, THREADS = 256, M = 8; };
 template <> struct LagTile<2, 3> { static constexpr int LX = 16, LY = 16, LZ = 1, THREADS = 256, M = 16; };
-template <> struct LagTile<1, 3> { static constexpr int LX = 128, LY = 1, LZ = 1, THREADS = 128, M = 32; };
 template <> struct LagTile<2, 0> { static constexpr int LX = 64, LY = 32, LZ = 1, THREADS = 512, M = 16; };
 template <> struct LagTile<2, 1> { static constexpr int LX = 32, LY = 16, LZ = 1, THREADS = 128, M = 16; };
 template <> struct LagTile<2, 2> { static constexpr int LX = 16, LY = 16, LZ = 1, THREADS = 64, M = 16; };
@@ -894,8 +893,12 @@ template <> struct LagTile<1, 2> { static constexpr int LX = 128, LY = 1, LZ = 1
 // Whether the LAG_SMALL tiles of np particles are one wave: four CTAs of 256
 // threads (64 registers each) on each of 148 SMs.
 template <int R> inline bool lag_small(size_t np) {
-    typedef LagTile<R, LAG_SMALL> L;
-    return R > 1 && np <= (size_t)(4 * 148) * (L::LX * L::LY * L::LZ);
+    if constexpr (R > 1) {
+        typedef LagTile<R, LAG_SMALL> L;
+        return np <= (size_t)(4 * 148) * (L::LX * L::LY * L::LZ);
+    } else {
+        return false;
+    }
 }
 
 // The body of the Lagrangian deposit for one lattice tile. FUSED: the
