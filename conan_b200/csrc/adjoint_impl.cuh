@@ -537,8 +537,7 @@ template <typename T, int R> struct Diff : DiffBase {
         CONAN_TRY(pm.alloc(&rhobar, pm.mf.cells));
         CONAN_TRY(pm.alloc(&S, 1));
         CONAN_TRY(pm.alloc(&absmax, 4 * ABS_SLOTS));
-        unsigned k = p.checkpoint_every ? p.checkpoint_every : 1;
-        for (unsigned i = 0; i <= p.n; i += k)
+        for (size_t i = 0; i < p.n; i += kev())  // the state before every kev()-th step
             for (int c = 0; c < 2 * R; ++c) {
                 T *b = nullptr;
                 CONAN_TRY(pm.alloc(&b, pm.np));

@@ -114,3 +114,19 @@ def test_captured_calls(gpu, conan, prec, mbits, n, every):
     torch.cuda.synchronize()
     del graphs, both, fwd, bwd
     m.close()
+
+
+def test_checkpoint_memory(gpu, conan):
+    """A slot per kept state and no more: 16 steps with a checkpoint every 8 keep two, as 15 steps do."""
+    from conan_b200.autograd import DiffPM
+    used = []
+    for n, every in ((8, 8), (15, 8), (16, 8), (16, 16), (8, 16), (16, 4)):  # the first loads the kernels
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        m = DiffPM(dim=3, mbits=7, L_box=60.0, ns=-2.0, a0=0.05, da=0.01, n=n, checkpoint_every=every)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        m.close()
+    slot = 6 * 4 * 128 ** 3
+    used = used[1:]
+    assert abs(used[1] - used[0]) < slot / 4 and abs(used[2] - used[3]) < slot / 4
+    assert abs(used[4] - used[1] - 2 * slot) < slot / 4 and abs(used[1] - used[2] - slot) < slot / 4
