@@ -338,13 +338,15 @@ __global__ void __launch_bounds__(256)
 // state back from s_{i+1} to s_i, using G = FD4 gradient at d_{i+1} and
 // rhobar = Green * div (null: zero); the maximum of the new |pbar| goes into
 // absmax (a pass of its own over pbar before: 160 us per step at 256^3).
-// Bound by the chain of its twelve streams and 16 corner loads: the register
-// budget of four blocks per SM takes 450 us at 256^3, three 547, five 524;
-// walking the lattice in 16 x 4 x 4 tiles 578 (half-used sectors of the
+// Bound by the chain of its twelve streams and 16 corner loads: in FP32 the
+// register budget of four blocks per SM takes 450 us at 256^3, three 547, five
+// 524. FP64 in 3D spills within four (84 bytes) and takes three: a backward of
+// four steps at 256^3 13.34 -> 12.90 ms (two 13.35), of eight at 128^3 3.92 ->
+// 3.80; 2D fits four. Walking the lattice in 16 x 4 x 4 tiles 578 (half-used sectors of the
 // streams cost more than the corner reads' locality gains), streaming loads
 // and stores 457.
 template <typename T, int R>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, sizeof(T) == 8 && R == 3 ? 3 : 4)
     k_adj_step(Parts<T> P, Mesh m, const G4<T> *__restrict__ G, const T *__restrict__ rhobar, T *pb0, T *pb1, T *pb2,
                T *db0, T *db1, T *db2, double ck, double cd, double mass, int periodic, unsigned long long *absmax) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
