@@ -496,8 +496,12 @@ template <typename T, int R> struct Diff : DiffBase {
     bool captured = false;
     // The launches of a pass between the caller's buffers, captured as graphs
     // from a handle's second pass on (a few microseconds of host time per
-    // launch, and there are hundreds; building a graph pays from the second
-    // use). Everything in them belongs to the handle.
+    // launch, and there are hundreds). Forward and backward by launches, in the
+    // pass that builds the graphs and by them: 32^3, 8 steps 1.61, 1.98, 1.01
+    // ms; 64^3, 10 steps 1.86, 2.15, 1.27; 128^3, 16 steps 7.3, 7.5, 6.3; 256^3,
+    // 6 steps 16.6, 16.7, 16.1: building costs at most two thirds of what each
+    // pass gains afterwards, and waits for the second since many handles make
+    // only one. Everything in them belongs to the handle.
     enum { G_STEPS, G_LAST, G_BACK, G_COUNT };
     cudaGraphExec_t graphs[G_COUNT] = {};
     unsigned graph_config = 0, passes[G_COUNT] = {};
@@ -773,9 +777,10 @@ template <typename T, int R> struct Diff : DiffBase {
     }
 
     // U = gather-transpose deposit of pb. The merging kernel needs whole warps
-    // within one member (8 particles per side) and, for its one-instruction rounding, a fixed-point
-    // exponent that leaves particles below 2^51 units: 2^18 particles are
-    // enough for both (and smaller lattices are launch-bound either way).
+    // within one member (8 particles per side) and, for its one-instruction
+    // rounding, a fixed-point exponent that leaves particles below 2^51 units:
+    // 2^18 particles are enough for both (and smaller lattices are launch-bound
+    // either way).
     int vec_deposit() {
         cudaStream_t st = pm.st;
         if (R > 1 && mm.n >= 8 && pm.np >= ((size_t)1 << 18)) {

@@ -791,8 +791,8 @@ static __global__ void __launch_bounds__(256) k_direct_mesh(ulonglong2 *__restri
 
 // Fused leapfrog update of particle i: the kick of Gravity::kick
 // (src/run/nbody.hh:112-117), then the next step's drift (Gravity::drift,
-// src/run/nbody.hh:122-130), then the counting-sort rank of the new cell.
-// or (FP64 with a direct accumulator dacc) the deposit of the new position.
+// src/run/nbody.hh:122-130), then either the counting-sort rank of the new cell
+// or, in FP64 with a direct accumulator dacc, the deposit of the new position.
 template <typename T, int R, bool SPECTRAL>
 __global__ void __launch_bounds__(256)
     k_gkd(Parts<T> P, Mesh m, const T *__restrict__ phi, const T *__restrict__ g0,
