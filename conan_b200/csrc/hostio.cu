@@ -130,11 +130,11 @@ int copy(void *host, void *devp, size_t bytes, bool to_host, cudaStream_t st) {
     // below four chunks the threads' start costs more than it saves (6 MB out
     // and in: 0.42 ms by the driver, 0.6 with three threads; 50 MB into fresh
     // pages 11 ms by the driver, 3.2 with eight)
-    const int dev = current_device();
-    const int cores = (int)std::thread::hardware_concurrency();
+    static const int cores = (int)std::thread::hardware_concurrency();  // a read of /sys
     const int want = (int)std::min<size_t>(std::min(HOSTIO_LANES, std::max(1, cores / 2)),
                                            bytes / HOSTIO_CHUNK);
-    if (dev >= 0 && want >= 4 && !page_locked(host)) {
+    const int dev = want >= 4 ? current_device() : -1;
+    if (dev >= 0 && !page_locked(host)) {
         std::vector<Lane> lanes = lanes_take(dev, want);
         if (lanes.size() >= 2) {
             cudaEvent_t after = nullptr;
