@@ -1127,7 +1127,9 @@ template <typename T, int R> struct PM : PMBase {
         if (dep_fits<0>()) cands.push_back({0, 0, "sorted 32x8x8 / 256 threads"});
         if (dep_fits<1>()) cands.push_back({0, 1, "sorted 32x4x8 / 128 threads"});
         if (dep_fits<2>()) cands.push_back({0, 2, "sorted 32x16x8 / 512 threads"});
-        if (dep_fits<DEP_SMALL>()) cands.push_back({0, DEP_SMALL, "sorted, tiles of 256 cells / 256 threads"});
+        // (where the large tiles fill the chip the small ones only cost tuning
+        // time: 128^3 FP32 13.4 against 12.4 ms)
+        if (dep_default() == DEP_SMALL) cands.push_back({0, DEP_SMALL, "sorted, tiles of 256 cells / 256 threads"});
         if (dacc) cands.push_back({0, DEP_DIRECT, "direct, two words per cell"});
         if (sizeof(T) == 4 && lacc) {
             const char *tile[4] = {"", "", "", ""};
