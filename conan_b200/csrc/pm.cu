@@ -568,7 +568,13 @@ template <typename T, int R> struct PM : PMBase {
     // mesh (unless the fused gather kernel did it already).
     int lag_accumulate() {
         if (!lag_ready) {
-            if (tma_ok && !pers_ok) {  // the staged tiles, neither kick nor drift
+            // The staged tiles (neither kick nor drift) where they have a full
+            // window: 256^3 512 -> 411 us, 128^3 70 -> 63 for displacements of
+            // three cells. The small tiles hide little behind one or two
+            // particles per thread (64^3 staged 20.4 us, old tiles 16.5), and
+            // with the two-cell window the momenta's loads are not worth the
+            // wait (256^3 f = 2 1050 against 955 us, 64^3 f = 4 50 against 48).
+            if (tma_ok && !pers_ok && lag_v != LAG_SMALL && lwin.w[0] > 2) {
                 const GKD c{0, 0, 0, 0, 0, 0};
                 CONAN_TRY(launch_gkd_lag(c, "deposit"));
             } else {
