@@ -721,14 +721,9 @@ template <typename T, int R> struct Diff : DiffBase {
         return forward_last();
     }
 
-    // After a pass that failed the solver's host state says nothing about what
-    // its launches left pending.
-    int failed(int rc) {
-        if (rc != CONAN_OK) pm.stale = true;
-        return rc;
-    }
     int forward(const void *noise, void *density, void *stream) override {
-        return failed(forward_pass(noise, density, stream));
+        const int rc = forward_pass(noise, density, stream);
+        return rc == CONAN_OK ? rc : pm.failed(rc);
     }
     int forward_pass(const void *noise, void *density, void *stream) {
         CONAN_TRY(enter(stream));
@@ -829,7 +824,8 @@ template <typename T, int R> struct Diff : DiffBase {
 
     int backward(const void *gdens, void *gnoise, void *stream) override {
         if (!have_forward) return set_error(CONAN_ERR_STATE, "backward without a forward call");
-        return failed(backward_pass(gdens, gnoise, stream));
+        const int rc = backward_pass(gdens, gnoise, stream);
+        return rc == CONAN_OK ? rc : pm.failed(rc);
     }
     int backward_pass(const void *gdens, void *gnoise, void *stream) {
         CONAN_TRY(enter(stream));

@@ -564,6 +564,20 @@ template <typename T, int R> struct PM : PMBase {
         return drop_lag_deposit();
     }
 
+    // After such a call: what it may have left is cleared before it returns (its
+    // message kept), since a graph that is replayed later asks no host flag.
+    // Within a caller's capture the next call on the host does that.
+    int failed(int rc) {
+        const std::string msg = last_error();
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        stale = true;
+        if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+            positions_reset() == CONAN_OK)
+            cudaStreamSynchronize(st);
+        last_error() = msg;
+        return rc;
+    }
+
     // The Lagrangian deposit of the current positions into the accumulator
     // mesh (unless the fused gather kernel did it already).
     int lag_accumulate() {
@@ -1447,13 +1461,7 @@ template <typename T, int R> struct PM : PMBase {
                 if (seg_end > n) seg_end = n;
             }
             const int rc = !prof.on && !debug_sync() ? graph_segment(a, da, i, seg_end) : steps(a, da, i, seg_end);
-            if (rc != CONAN_OK) {
-                const std::string msg = last_error();
-                stale = true;
-                positions_reset();
-                last_error() = msg;
-                return rc;
-            }
+            if (rc != CONAN_OK) return failed(rc);
             i = seg_end;
             if (cb) {
                 CONAN_CUDA(cudaStreamSynchronize(st));

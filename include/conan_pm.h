@@ -218,8 +218,8 @@ int conan_pm_kick(conan_pm *h, double a, double da);
 typedef int (*conan_step_cb)(conan_pm *h, unsigned step, double a, void *user);
 
 /* The callback of conan_pm_run fires after steps with (i+1) % k == 0 and
- * after the last step (default k = 1). Steps between callbacks run as one
- * CUDA graph with the kick of one step fused to the drift of the next. */
+ * after the last step (default k = 1). Steps between callbacks run as
+ * CUDA graphs with the kick of one step fused to the drift of the next. */
 int conan_pm_set_callback_interval(conan_pm *h, unsigned k);
 
 /* Deposit algorithm of the handle (both give the same density, bit for bit,

@@ -98,6 +98,28 @@ def test_model_pass_that_fails(gpu, conan, monkeypatch, prec, mbits, plane, fail
     m.close()
 
 
+def test_ensemble_run_after_a_failed_pass(gpu, conan, monkeypatch):
+    """The run is one graph that is replayed: the deposit that the failed pass left
+    for its plane transform is gone before."""
+    from conan_b200 import _lib as L
+    from conan_b200.ensemble import Ensemble
+    monkeypatch.setenv("CONAN_PLANE_PASS", "2")
+    e = Ensemble([(8, 100.0, -2.0, 1)], a0=0.05, a_end=0.15, steps=2, autotune=False)
+    e.init()
+    e.run()
+    want = [x.copy() for x in e.state(0)]
+    try:
+        L.lib().conan_selftest_fail_graph(1)  # the model's second pass: its last step's graph
+        with pytest.raises(conan.ConanError):
+            e.forward_adjoint()
+    finally:
+        L.lib().conan_selftest_fail_graph(-1)
+    e.run()
+    for a, b in zip(e.state(0), want):
+        assert np.array_equal(a, b)
+    e.close()
+
+
 def test_handles_get_the_memory_that_calls_without_one_keep(gpu, conan):
     """A friends-of-friends handle of 0.6 GB and the autotuner's copy of a state
     beside an array that leaves less free than they need: what a field call of
